@@ -12,20 +12,21 @@
 //      sources coincide at 2^-21 L;
 //   4. node mass and COM from exact 64-bit prefix sums of 2^-40 L fixed-point
 //      coordinates (no summation-order error).
-// Walk: one warp per 32 targets (sorted by key, so a warp's targets are close).
-// The warp traverses a shared depth-first stack; each lane classifies the node
-// against its target -- pruned (cube outside the cutoff sphere), leaf (exact
-// pairs), monopole (modified Barnes-Hut criterion, not containing the target,
-// not straddling the cutoff) or open -- and the node's children are pushed if
-// any lane needs them. A lane that pruned or accepted a node records its end
-// index and ignores that node's descendants, which follow it contiguously in
-// depth-first order. Stack depth and iterations are bounded; overflow is an
-// error status, never an unbounded loop.
+// Walk: one warp per group of G targets (G of 1, 8, 16 or 32, neighbours in key
+// order). The 32 lanes classify 32 nodes at a time against the group's bounding
+// box: dropped for every target, opened for every target, a monopole for every
+// target, or undecided, in which case each target decides for itself in
+// binary64. Sources and accepted monopoles collect in a shared-memory list that
+// every target then filters by distance and sums. Each target's set of exact
+// pairs and monopoles is the one of the reference's per-target walk. Stack depth
+// and iterations are bounded; overflow is an error status, never an unbounded
+// loop.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <new>
 #include <string>
 #include <vector>
@@ -42,7 +43,10 @@ namespace {
 
 constexpr int kT = 256;
 constexpr int kBits = 21;
-constexpr int kStack = 192;        // per-warp stack entries (>= 7 * 21 + 8)
+// Per-warp stack of unopened child runs. Above kStackWide entries one run is
+// popped at a time, so the stack stays within kStackWide + 31 + 7 * 21 + 8 entries.
+constexpr int kStack = 320;
+constexpr int kStackWide = 128;
 constexpr unsigned kMaxIter = 1u << 24;
 
 inline unsigned nb(uint64_t n, int t = kT) { return static_cast<unsigned>((n + t - 1) / t); }
@@ -331,68 +335,225 @@ __device__ __forceinline__ double min_image(double d, double L) {
 }
 
 struct WalkParams {
-    double L, r_cut, eps, theta, r_s, G, m;
+    double L, r_cut, eps, r_s, G, m;
 };
 
-// The monopole criterion's target-independent side, once per node: a node is
-// accepted when its COM distance squared exceeds (2 half / theta + off)^2
-// with off the L1 offset of the COM from the cube centre (the expression the
-// walk would otherwise evaluate at every visit, in the same operations).
-__global__ void k_open_radius(uint32_t n_nodes, double theta, Node* __restrict__ nodes) {
+constexpr unsigned kCounters = 64;   // pairs of walk statistics counters
+
+// Box coordinates as 32-bit fractions of L: differences wrap like the box does,
+// so the signed difference is the minimum image.
+__device__ __forceinline__ uint32_t box_fraction(double v, double L) {
+    return __double2uint_rz(v * (4294967296.0 / L));   // saturates
+}
+
+// What the group tests of the walk read of a node, once after the build, in
+// three 16-byte arrays that the lanes of a warp read as short runs (the children
+// of a node are consecutive):
+//   ga  cube centre and half side, in 2^-32 L (both exact)
+//   gm  centre of mass in 2^-32 L, and the square of the opening distance in
+//       the same unit (float bits)
+//   gc  first child, children | leaf << 8, source range start and count
+// The monopole criterion's target-independent side is open2: a node is accepted
+// when its COM distance squared exceeds (2 half / theta + off)^2 with off the L1
+// offset of the COM from the cube centre.
+__global__ void k_walk_nodes(uint32_t n_nodes, double theta, double L, Node* __restrict__ nodes,
+                             uint4* __restrict__ ga, uint4* __restrict__ gm,
+                             uint4* __restrict__ gc) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_nodes) return;
     Node& nd = nodes[i];
     const double off = fabs(nd.mx - nd.cx) + fabs(nd.my - nd.cy) + fabs(nd.mz - nd.cz);
     const double need = 2.0 * nd.half / theta + off;
     nd.open2 = need * need;
+    const double unit = 4294967296.0 / L;
+    const float need_u = static_cast<float>(need * unit);
+    ga[i] = make_uint4(box_fraction(nd.cx, L), box_fraction(nd.cy, L), box_fraction(nd.cz, L),
+                       0x80000000u >> nd.level);
+    gm[i] = make_uint4(box_fraction(nd.mx, L), box_fraction(nd.my, L), box_fraction(nd.mz, L),
+                       __float_as_uint(need_u * need_u));
+    gc[i] = make_uint4(nd.first_child, nd.n_child | (nd.leaf << 8), nd.start, nd.end - nd.start);
+}
+
+// The pair factor as A^3 - h, A = (r^2 + eps^2)^(-1/2), with the long-range part
+//   h(r^2) = (1 - M_S(q)) / r^3 = r_s^-3 sum_k (-1)^k q^(2k) 2(k+1) / ((2k+3) 4^(k+1) (k+1)! sqrt(pi)),
+// an entire function of t = q^2, as one polynomial in tau = 2 t / t_max - 1 over
+// the whole cutoff sphere (pair_poly, below): no branch, no error function, no
+// exponential. One rsqrt and DEG + 8 multiply-adds replace the erfc, exp, expm1,
+// log1p, sqrt and division of short_factor_impl, which remains for cutoffs of so
+// many r_s that no polynomial of these degrees reaches the accuracy (DEG = 0).
+constexpr int kDegLow = 12, kDegMid = 20, kDegHigh = 28;
+struct PairPoly {
+    double tau;                 // 2 / (t_max r_s^2)
+    double c[kDegHigh + 1];     // monomial coefficients in tau, times r_s^-3
+};
+
+template <typename R, int DEG>
+__device__ __forceinline__ double pair_factor(double r2, double eps2, double inv_rs,
+                                              const PairPoly& pp) {
+    if constexpr (DEG == 0) {
+        const R irs = static_cast<R>(inv_rs);
+        return static_cast<double>(short_factor_impl<R>(static_cast<R>(r2), static_cast<R>(eps2),
+                                                        irs, irs * irs * irs));
+    } else {
+        const double tau = r2 * pp.tau - 1.0;
+        const double t2 = tau * tau;
+        double even = pp.c[DEG], odd = pp.c[DEG - 1];
+#pragma unroll
+        for (int k = DEG - 2; k >= 0; k -= 2) {
+            even = even * t2 + pp.c[k];
+            if (k > 0) odd = odd * t2 + pp.c[k - 1];
+        }
+        const double s = r2 + eps2;
+        double a;
+        if constexpr (sizeof(R) == 8) {
+            a = rsqrt(s);
+        } else {
+            // the FP32 reciprocal square root and one Newton step: 2e-14
+            a = static_cast<double>(rsqrtf(static_cast<float>(s)));
+            a = a * (1.5 - 0.5 * s * a * a);
+        }
+        return a * a * a - (odd * tau + even);
+    }
 }
 
 // Targets: sorted slots tslot[t] (null: target t is sorted slot t, every
 // source). Output of target t goes to index out_idx[t] (null: t), written, or
 // added to what is there when `add`. Source masses: sorted sm[] (null: P.m).
 //
-// Blocks per SM the registers are sized for. The binary64 walk waits mostly on
-// the FP64 pipe's fixed latencies, which more warps hide: eight 128-thread
-// blocks (64 registers, 52 bytes of spill) against the compiler's five (88
-// registers) took the c5 walk from 1444 to 1283 ms. The FP32 walk measured
-// 863 ms at the compiler's 71 registers (seven blocks), 874 at eight blocks and
-// 879 at six, so it keeps its own choice.
-#ifndef HYOWON_WALK_MINB64
-#define HYOWON_WALK_MINB64 8
-#endif
-#ifndef HYOWON_WALK_MINB32
-#define HYOWON_WALK_MINB32 1
-#endif
-template <typename R> struct WalkBlocks {
-    static constexpr int minb = sizeof(R) == 8 ? HYOWON_WALK_MINB64 : HYOWON_WALK_MINB32;
+// One warp per block and group of G targets; lane l works for target l % G and
+// takes every (32 / G)-th list entry. What bounds it: instruction issue, shared
+// between the pair factors (FP64), the distance filter and the node tests. A walk
+// with one lane per target ran with 11 of 32 lanes active, and each lane
+// classified every node its warp reached in binary64; here a node costs one lane a
+// few integer and FP32 operations for the whole group.
+// 24 warps per SM (80 registers, no spill in the forms that run): 28 and 20 measured
+// 34.2 / 33.6 / 34.8 ms on 2.1M clustered sources at G = 16.
+constexpr int kWalkWarps = 24;
+template <int G>
+struct WalkShape {
+    static constexpr int S = 32 / G;                  // lanes per target
+    static constexpr int cap = S < 4 ? 32 * S : 128;  // list entries, >= 32
+    static constexpr int per_lane = cap / S;          // one bit each of a 32-bit word
+    static_assert(per_lane <= 32 && cap >= 32, "list layout");
 };
-template <typename R>
-__global__ void __launch_bounds__(128, WalkBlocks<R>::minb)
+
+template <typename R, int DEG, int G>
+__global__ void __launch_bounds__(32, kWalkWarps)
 k_walk(uint32_t n_targets, const uint32_t* __restrict__ tslot, const double* __restrict__ sx,
        const double* __restrict__ sy, const double* __restrict__ sz,
        const double* __restrict__ sm, const unsigned long long* __restrict__ skey,
-       const Node* __restrict__ nodes, uint32_t n_nodes, WalkParams P,
-       const uint32_t* __restrict__ out_idx, int add, double* __restrict__ ax,
+       const Node* __restrict__ nodes, const uint4* __restrict__ ga,
+       const uint4* __restrict__ gm, const uint4* __restrict__ gc, uint32_t n_nodes, WalkParams P,
+       const PairPoly pp, const uint32_t* __restrict__ out_idx, int add, double* __restrict__ ax,
        double* __restrict__ ay, double* __restrict__ az,
        unsigned long long* __restrict__ counters, unsigned int* status) {
-    __shared__ uint32_t stack[4][kStack];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t t = (blockIdx.x * 4 + warp) * 32 + lane;
-    const bool valid = t < n_targets;
-    uint32_t slot = valid ? (tslot ? tslot[t] : t) : 0u;
+    using Shape = WalkShape<G>;
+    constexpr int S = Shape::S, CAP = Shape::cap, PER = Shape::per_lane;
+    constexpr uint32_t kGroup = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+    constexpr unsigned kAll = 0xffffffffu;
+    __shared__ double ex[CAP], ey[CAP], ez[CAP], ew[CAP];  // entry position (the group's image), G m
+    __shared__ float4 erel[CAP];              // (position - group centre) / r_cut, target mask
+    __shared__ float4 ucell[32], ucom[32];    // undecided nodes: cube centre, half; COM, opening
+    __shared__ uint32_t unode[32], umask[32], uaccept[32], uopen[32];
+    __shared__ uint32_t gfirst[32], gsource[32], gnode[32], gmono[32], gopen[32];
+    __shared__ uint32_t run_first[kStack], run_count[kStack], run_mask[kStack];
+    const int lane = threadIdx.x;
+    const int t = lane % G, sub = lane / G;
+    const unsigned below = (1u << lane) - 1u;
+    const uint32_t t0 = blockIdx.x * G;
+    const uint32_t n_here = n_targets - t0 < G ? n_targets - t0 : G;
+    const bool valid = static_cast<uint32_t>(t) < n_here;
+    const uint32_t ti = t0 + (valid ? t : 0u);
+    const uint32_t slot = tslot ? tslot[ti] : ti;
     const double tx = sx[slot], ty = sy[slot], tz = sz[slot];
-    const unsigned long long tkey = skey[slot];
-    const R eps2 = static_cast<R>(P.eps * P.eps);
-    const R inv_rs = static_cast<R>(1.0 / P.r_s);
-    const R inv_rs3 = inv_rs * inv_rs * inv_rs;
-    const double rc2 = P.r_cut * P.r_cut;
-    R fx = 0, fy = 0, fz = 0;
-    uint32_t skip_end = valid ? 0u : 0xffffffffu;
-    unsigned long long visits = 0, pairs = 0;
-    uint32_t* st = stack[warp];
-    int sp = 0;
-    if (lane == 0) st[0] = 0;
-    sp = 1;
+
+    // The group's bounding box in 2^-32 L: centre, and half sides with slack for
+    // the rounding of positions and centres of mass to that unit. safe: every
+    // source within r_cut of a target lies in the image nearest to the centre.
+    // inner: in the image it is stored in.
+    uint32_t gcu[3], ge[3];
+    double ctr[3];
+    bool safe = true, inner = true;
+    const float unit_rc = static_cast<float>(P.r_cut * (4294967296.0 / P.L));
+    const float inv_unit = 1.f / unit_rc;
+    const double inv_rc = 1.0 / P.r_cut;
+    float er[3], e_max = 0.f;   // half sides over r_cut
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const uint32_t u = box_fraction(a == 0 ? tx : (a == 1 ? ty : tz), P.L);
+        const uint32_t lo = __reduce_min_sync(kAll, u), hi = __reduce_max_sync(kAll, u);
+        gcu[a] = lo + (hi - lo) / 2;
+        ge[a] = (hi - lo) / 2 + 4u;
+        ctr[a] = gcu[a] * (P.L / 4294967296.0);
+        const float span = unit_rc * 1.000001f + 2.f * static_cast<float>(ge[a]);
+        safe = safe && span < 2147483000.f;
+        inner = inner && static_cast<float>(lo) > unit_rc * 1.00001f + 1024.f
+            && static_cast<float>(hi) < 4294966000.f - unit_rc * 1.00001f;
+        er[a] = static_cast<float>(ge[a]) * inv_unit;
+        e_max = fmaxf(e_max, er[a]);
+    }
+    inner = inner && safe;
+    const float rc2 = unit_rc * unit_rc;
+    const float rc2_hi = rc2 * 1.00001f, rc2_lo = rc2 * 0.99999f;
+    // slack of FP32 coordinates relative to the centre, in units of r_cut
+    // (magnitudes up to 2 + 2 e / r_cut, and 4 units of 2^-32 L)
+    const float slack = 4e-7f * (2.f + 2.f * e_max) + 4.f * inv_unit;
+    const float cut_hi = (1.f + 2.f * slack) * (1.f + 2.f * slack);
+    const float cut_lo = (1.f - 2.f * slack) * (1.f - 2.f * slack);
+    const float frx = static_cast<float>((tx - ctr[0]) * inv_rc);
+    const float fry = static_cast<float>((ty - ctr[1]) * inv_rc);
+    const float frz = static_cast<float>((tz - ctr[2]) * inv_rc);
+    const double eps2 = P.eps * P.eps, inv_rs = 1.0 / P.r_s, rcut2 = P.r_cut * P.r_cut;
+
+    const float reach2 = safe ? cut_hi : __int_as_float(0x7f800000);   // unsafe: no filter
+    const uint32_t tbit = 1u << t;
+
+    double fx = 0.0, fy = 0.0, fz = 0.0;
+    uint32_t visits = 0, pairs = 0;
+    int count = 0;   // entries in the list
+
+    // Every target sums the listed entries: a distance filter into one bit per
+    // entry, then the pair factor over the set bits.
+    auto flush = [&]() {
+        __syncwarp();
+        // stale entries of a part-filled list belong to nobody
+        for (int e = count + lane; e < CAP; e += 32) erel[e].w = 0.f;
+        __syncwarp();
+        uint32_t bits = 0;
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+            const float4 c = erel[k * S + sub];
+            const float dx = c.x - frx, dy = c.y - fry, dz = c.z - frz;
+            if (dx * dx + dy * dy + dz * dz < reach2 && (__float_as_uint(c.w) & tbit)) bits |= 1u << k;
+        }
+        while (bits) {
+            const int e = (__ffs(bits) - 1) * S + sub;
+            bits &= bits - 1;
+            double dx = ex[e] - tx, dy = ey[e] - ty, dz = ez[e] - tz;
+            if (!safe) {
+                dx = min_image(dx, P.L);
+                dy = min_image(dy, P.L);
+                dz = min_image(dz, P.L);
+            }
+            const double r2 = dx * dx + dy * dy + dz * dz;
+            if (r2 < rcut2 && r2 != 0.0) {   // 0: the target itself
+                const double f = pair_factor<R, DEG>(r2, eps2, inv_rs, pp) * ew[e];
+                fx += f * dx;
+                fy += f * dy;
+                fz += f * dz;
+                ++pairs;
+            }
+        }
+        __syncwarp();
+        count = 0;
+    };
+
+    if (lane == 0) {
+        run_first[0] = 0;
+        run_count[0] = 1;
+        run_mask[0] = n_here == 32u ? kAll : (1u << n_here) - 1u;
+    }
+    int sp = 1;
     __syncwarp();
     unsigned iter = 0;
     while (sp > 0) {
@@ -400,110 +561,353 @@ k_walk(uint32_t n_targets, const uint32_t* __restrict__ tslot, const double* __r
             if (lane == 0) raise_status(status, ST_CAPACITY);
             break;
         }
-        const uint32_t ni = st[sp - 1];
-        --sp;
+        // Pop child runs from the top, as many as give at most 32 nodes.
+        uint32_t pop_first = 0, pop_n = 0, pop_mask = 0;
+        if (lane < sp && (lane == 0 || sp <= kStackWide)) {
+            pop_first = run_first[sp - 1 - lane];
+            pop_n = run_count[sp - 1 - lane];
+            pop_mask = run_mask[sp - 1 - lane];
+        }
+        uint32_t inc = pop_n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(kAll, inc, o);
+            if (lane >= o) inc += v;
+        }
+        const uint32_t exc = inc - pop_n;
+        const bool taken = pop_n > 0 && inc <= 32u;
+        const int runs = __popc(__ballot_sync(kAll, taken));
+        const unsigned starts = __reduce_or_sync(kAll, taken ? 1u << exc : 0u);
+        const uint32_t total = __shfl_sync(kAll, inc, runs - 1);
+        const int from = __popc(starts & (below | (1u << lane))) - 1;
+        const uint32_t ni = __shfl_sync(kAll, pop_first - exc, from) + static_cast<uint32_t>(lane);
+        uint32_t mask = __shfl_sync(kAll, pop_mask, from);
+        const bool active = static_cast<uint32_t>(lane) < total;
+        sp -= runs;
+        if (runs == 0 || __any_sync(kAll, active && ni >= n_nodes)) {
+            if (lane == 0) raise_status(status, ST_CELL_ESCAPE);
+            break;
+        }
         __syncwarp();
-        const Node nd = nodes[ni];
-        bool need_open = false;
-        if (nd.start >= skip_end) {
-            ++visits;
-            // cube vs cutoff sphere (minimum image of the centre)
-            const double dcx = min_image(nd.cx - tx, P.L), dcy = min_image(nd.cy - ty, P.L),
-                         dcz = min_image(nd.cz - tz, P.L);
-            const double h = nd.half;
-            int rel;
-            if (h >= 0.25 * P.L) {
-                rel = 0;
+
+        // Classify node ni for the whole group. am: targets that take its
+        // monopole; om: targets that need its children (a leaf's sources).
+        uint32_t am = 0, om = 0;
+        uint4 link = make_uint4(0, 0, 0, 0);
+        bool undecided = false;
+        float4 cell, com;
+        if (active) {
+            visits += __popc(mask);
+            const uint4 a = ga[ni];
+            link = gc[ni];
+            const uint32_t h = a.w;
+            const int d[3] = {static_cast<int>(a.x - gcu[0]), static_cast<int>(a.y - gcu[1]),
+                              static_cast<int>(a.z - gcu[2])};
+            if (h >= 0x40000000u) {
+                om = mask;   // a quarter of the box or more: always opened
             } else {
-                const double ex = fmax(fabs(dcx) - h, 0.0), ey = fmax(fabs(dcy) - h, 0.0),
-                             ez = fmax(fabs(dcz) - h, 0.0);
-                const double fx2 = fabs(dcx) + h, fy2 = fabs(dcy) + h, fz2 = fabs(dcz) + h;
-                if (ex * ex + ey * ey + ez * ez >= rc2) rel = -1;
-                else if (fx2 * fx2 + fy2 * fy2 + fz2 * fz2 < rc2) rel = 1;
-                else rel = 0;
-            }
-            if (rel < 0) {
-                skip_end = nd.end;
-            } else if (nd.leaf) {
-                for (uint32_t i = nd.start; i < nd.end; ++i) {
-                    if (i == slot) continue;
-                    const double dx = min_image(sx[i] - tx, P.L), dy = min_image(sy[i] - ty, P.L),
-                                 dz = min_image(sz[i] - tz, P.L);
-                    const double r2 = dx * dx + dy * dy + dz * dz;
-                    if (!(r2 < rc2) || r2 == 0.0) continue;
-                    const R f = short_factor_impl<R>(static_cast<R>(r2), eps2, inv_rs, inv_rs3)
-                        * static_cast<R>(P.G * (sm ? sm[i] : P.m));
-                    fx += f * static_cast<R>(dx);
-                    fy += f * static_cast<R>(dy);
-                    fz += f * static_cast<R>(dz);
-                    ++pairs;
+                float near2 = 0.f, lo2 = 0.f, far2 = 0.f;
+                bool apart = false;
+                const float hf = static_cast<float>(h);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    const uint32_t D = static_cast<uint32_t>(abs(d[k]));
+                    const uint32_t low = D > ge[k] ? D - ge[k] : 0u;
+                    const uint32_t gap = low > h ? low - h : 0u;
+                    apart = apart || gap > 8u;
+                    const float g = static_cast<float>(gap), l = static_cast<float>(low) + hf,
+                                f = static_cast<float>(D) + static_cast<float>(ge[k]) + hf;
+                    near2 += g * g;
+                    lo2 += l * l;
+                    far2 += f * f;
                 }
-                skip_end = nd.end;
-            } else {
-                const int shift = 3 * (kBits - static_cast<int>(nd.level));
-                const bool contains = shift >= 64 ? true : ((tkey >> shift) == nd.prefix);
-                bool accept = false;
-                double dx = 0, dy = 0, dz = 0, r2 = 0;
-                if (!contains && rel > 0) {
-                    dx = min_image(nd.mx - tx, P.L);
-                    dy = min_image(nd.my - ty, P.L);
-                    dz = min_image(nd.mz - tz, P.L);
-                    r2 = dx * dx + dy * dy + dz * dz;
-                    accept = r2 > nd.open2;
-                }
-                if (accept) {
-                    const R f = short_factor_impl<R>(static_cast<R>(r2), eps2, inv_rs, inv_rs3)
-                        * static_cast<R>(P.G * nd.mass);
-                    fx += f * static_cast<R>(dx);
-                    fy += f * static_cast<R>(dy);
-                    fz += f * static_cast<R>(dz);
-                    ++pairs;
-                    skip_end = nd.end;
-                } else {
-                    need_open = true;
+                if (near2 < rc2_hi) {   // else outside every target's cutoff sphere
+                    const bool leaf = (link.y >> 8) != 0;
+                    om = mask;          // a leaf, or a node inside nobody's sphere
+                    if (!leaf && lo2 < rc2_hi) {
+                        const uint4 m = gm[ni];
+                        const float open2 = __uint_as_float(m.w);
+                        const int c[3] = {static_cast<int>(m.x - gcu[0]),
+                                          static_cast<int>(m.y - gcu[1]),
+                                          static_cast<int>(m.z - gcu[2])};
+                        float min2 = 0.f, max2 = 0.f;
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) {
+                            const uint32_t M = static_cast<uint32_t>(abs(c[k]));
+                            const float l = static_cast<float>(M > ge[k] ? M - ge[k] : 0u);
+                            const float f = static_cast<float>(M) + static_cast<float>(ge[k]);
+                            min2 += l * l;
+                            max2 += f * f;
+                        }
+                        if (open2 < rc2_hi && max2 > open2 * 0.99999f) {
+                            om = 0;
+                            if (apart && far2 < rc2_lo && min2 > open2 * 1.00001f) {
+                                am = mask;
+                            } else {
+                                undecided = true;
+                                cell = make_float4(d[0] * inv_unit, d[1] * inv_unit,
+                                                   d[2] * inv_unit, hf * inv_unit);
+                                com = make_float4(c[0] * inv_unit, c[1] * inv_unit,
+                                                  c[2] * inv_unit, sqrtf(open2) * inv_unit);
+                            }
+                        }
+                    }
                 }
             }
         }
-        const unsigned open = __ballot_sync(0xffffffffu, need_open);
-        if (open) {
-            if (nd.first_child >= n_nodes || nd.n_child > n_nodes - nd.first_child) {
-                if (lane == 0) raise_status(status, ST_CELL_ESCAPE);
-                break;
+
+        // Undecided nodes, S at a time: each target applies the criterion itself,
+        // in FP32 relative to the group's centre where that settles it, else with
+        // the reference's binary64 expressions.
+        const unsigned todo = __ballot_sync(kAll, undecided);
+        if (todo) {
+            const int n_todo = __popc(todo), at = __popc(todo & below);
+            if (undecided) {
+                ucell[at] = cell;
+                ucom[at] = com;
+                unode[at] = ni;
+                umask[at] = mask;
             }
-            if (sp + static_cast<int>(nd.n_child) > kStack) {
-                if (lane == 0) raise_status(status, ST_CAPACITY);
-                break;
+            __syncwarp();
+            for (int b = 0; b < n_todo; b += S) {
+                const int u = b + sub;
+                bool accept = false, open = false;
+                if (u < n_todo && ((umask[u] >> t) & 1u)) {
+                    const float4 c = ucell[u], m = ucom[u];
+                    const float dx = fabsf(c.x - frx), dy = fabsf(c.y - fry),
+                                dz = fabsf(c.z - frz);
+                    const float nx = fmaxf(dx - c.w, 0.f), ny = fmaxf(dy - c.w, 0.f),
+                                nz = fmaxf(dz - c.w, 0.f);
+                    const float gx = dx + c.w, gy = dy + c.w, gz = dz + c.w;
+                    const float far2 = gx * gx + gy * gy + gz * gz;
+                    const float mx = m.x - frx, my = m.y - fry, mz = m.z - frz;
+                    const float r2 = mx * mx + my * my + mz * mz;
+                    const float hi = m.w * 1.000001f + 2.f * slack;
+                    const float lo = fmaxf(m.w * 0.999999f - 2.f * slack, 0.f);
+                    const bool apart = fmaxf(nx, fmaxf(ny, nz)) > 2.f * slack;
+                    // opening a node just outside the cutoff changes nothing: the
+                    // sources below it are rejected by their own distances
+                    open = nx * nx + ny * ny + nz * nz < cut_hi;
+                    const bool maybe = !safe || (open && far2 < cut_hi && r2 > lo * lo);
+                    accept = safe && maybe && apart && far2 < cut_lo && r2 > hi * hi;
+                    if (maybe && !accept) {
+                        const Node& nd = nodes[unode[u]];
+                        const double dcx = fabs(min_image(nd.cx - tx, P.L)),
+                                     dcy = fabs(min_image(nd.cy - ty, P.L)),
+                                     dcz = fabs(min_image(nd.cz - tz, P.L));
+                        const double h = nd.half;
+                        const double qx = fmax(dcx - h, 0.0), qy = fmax(dcy - h, 0.0),
+                                     qz = fmax(dcz - h, 0.0);
+                        const double sx2 = dcx + h, sy2 = dcy + h, sz2 = dcz + h;
+                        open = qx * qx + qy * qy + qz * qz < rcut2;
+                        const int shift = 3 * (kBits - static_cast<int>(nd.level));
+                        const bool contains = shift >= 64 || (skey[slot] >> shift) == nd.prefix;
+                        if (open && !contains && sx2 * sx2 + sy2 * sy2 + sz2 * sz2 < rcut2) {
+                            const double ox = min_image(nd.mx - tx, P.L),
+                                         oy = min_image(nd.my - ty, P.L),
+                                         oz = min_image(nd.mz - tz, P.L);
+                            accept = ox * ox + oy * oy + oz * oz > nd.open2;
+                        }
+                    }
+                    open = open && !accept;
+                }
+                const unsigned acc = __ballot_sync(kAll, accept), opn = __ballot_sync(kAll, open);
+                if (t == 0 && u < n_todo) {
+                    uaccept[u] = (acc >> (sub * G)) & kGroup;
+                    uopen[u] = (opn >> (sub * G)) & kGroup;
+                }
             }
-            if (lane == 0) {
-                for (uint32_t c = 0; c < nd.n_child; ++c)
-                    st[sp + c] = nd.first_child + nd.n_child - 1 - c;
+            __syncwarp();
+            if (undecided) {
+                am = uaccept[at];
+                om = uopen[at];
             }
-            sp += static_cast<int>(nd.n_child);
             __syncwarp();
         }
+
+        // Push the opened nodes' children; when every child holds one source,
+        // and for a leaf, the sources join the list instead.
+        const uint32_t n_child = link.y & 0xffu;
+        const bool direct = om != 0 && ((link.y >> 8) != 0 || n_child == link.w);
+        const bool push = om != 0 && !direct;
+        const unsigned pushes = __ballot_sync(kAll, push);
+        if (sp + __popc(pushes) > kStack || __any_sync(kAll, push && n_child > 8u)) {
+            if (lane == 0) raise_status(status, n_child > 8u ? ST_CELL_ESCAPE : ST_CAPACITY);
+            break;
+        }
+        if (push) {
+            const int at = sp + __popc(pushes & below);
+            run_first[at] = link.x;
+            run_count[at] = n_child;
+            run_mask[at] = om;
+        }
+        sp += __popc(pushes);
+
+        // The list items of this step (a monopole and / or a source range per
+        // lane), numbered across the warp and taken 32 at a time, one per lane.
+        const uint32_t mono = am != 0 ? 1u : 0u;
+        const uint32_t items = mono + (direct ? link.w : 0u);
+        const unsigned givers = __ballot_sync(kAll, items != 0);
+        if (givers) {
+            uint32_t upto = items;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(kAll, upto, o);
+                if (lane >= o) upto += v;
+            }
+            const uint32_t n_items = __shfl_sync(kAll, upto, 31), first = upto - items;
+            if (items) {
+                const int at = __popc(givers & below);
+                gfirst[at] = first + mono;           // number of the first source
+                gsource[at] = link.z;
+                gnode[at] = ni;
+                gmono[at] = am;
+                gopen[at] = om;
+            }
+            __syncwarp();
+            int before = 0;   // givers that start before the 32 items at hand
+            for (uint32_t base = 0; base < n_items; base += 32) {
+                const bool here = items && first >= base && first < base + 32;
+                const unsigned starts_here = __reduce_or_sync(kAll, here ? 1u << (first - base) : 0u);
+                const uint32_t i = base + static_cast<uint32_t>(lane);
+                bool have = i < n_items;
+                double x = 0.0, y = 0.0, z = 0.0, w = 0.0;
+                float rx = 0.f, ry = 0.f, rz = 0.f;
+                uint32_t who = 0;
+                if (have) {
+                    const int g = before + __popc(starts_here & (below | (1u << lane))) - 1;
+                    const uint32_t f = gfirst[g];
+                    if (i < f) {
+                        const Node& nd = nodes[gnode[g]];
+                        x = nd.mx;
+                        y = nd.my;
+                        z = nd.mz;
+                        w = P.G * nd.mass;
+                        who = gmono[g];
+                    } else {
+                        const uint32_t j = gsource[g] + (i - f);
+                        x = sx[j];
+                        y = sy[j];
+                        z = sz[j];
+                        w = P.G * (sm ? sm[j] : P.m);
+                        who = gopen[g];
+                    }
+                    if (safe && !inner) {   // the image nearest to the centre
+                        const double half = 0.5 * P.L;
+                        if (x - ctr[0] > half) x -= P.L;
+                        else if (x - ctr[0] < -half) x += P.L;
+                        if (y - ctr[1] > half) y -= P.L;
+                        else if (y - ctr[1] < -half) y += P.L;
+                        if (z - ctr[2] > half) z -= P.L;
+                        else if (z - ctr[2] < -half) z += P.L;
+                    }
+                    rx = static_cast<float>((x - ctr[0]) * inv_rc);
+                    ry = static_cast<float>((y - ctr[1]) * inv_rc);
+                    rz = static_cast<float>((z - ctr[2]) * inv_rc);
+                    if (safe) {   // within reach of the group's box
+                        const float qx = fmaxf(fabsf(rx) - er[0], 0.f),
+                                    qy = fmaxf(fabsf(ry) - er[1], 0.f),
+                                    qz = fmaxf(fabsf(rz) - er[2], 0.f);
+                        have = qx * qx + qy * qy + qz * qz < cut_hi;
+                    }
+                }
+                before += __popc(starts_here);
+                const unsigned all = __ballot_sync(kAll, have);
+                const int more = __popc(all);
+                if (count + more > CAP) flush();
+                if (have) {
+                    const int e = count + __popc(all & below);
+                    ex[e] = x;
+                    ey[e] = y;
+                    ez[e] = z;
+                    ew[e] = w;
+                    erel[e] = make_float4(rx, ry, rz, __uint_as_float(who));
+                }
+                count += more;
+            }
+        }
+        __syncwarp();
     }
-    if (valid) {
-        const uint32_t o = out_idx ? out_idx[t] : t;
+    if (count) flush();
+#pragma unroll
+    for (int o = G; o < 32; o <<= 1) {   // the lanes of one target
+        fx += __shfl_xor_sync(kAll, fx, o);
+        fy += __shfl_xor_sync(kAll, fy, o);
+        fz += __shfl_xor_sync(kAll, fz, o);
+    }
+    if (valid && sub == 0) {
+        const uint32_t o = out_idx ? out_idx[ti] : ti;
         if (add) {
-            ax[o] += static_cast<double>(fx);
-            ay[o] += static_cast<double>(fy);
-            az[o] += static_cast<double>(fz);
+            ax[o] += fx;
+            ay[o] += fy;
+            az[o] += fz;
         } else {
-            ax[o] = static_cast<double>(fx);
-            ay[o] = static_cast<double>(fy);
-            az[o] = static_cast<double>(fz);
+            ax[o] = fx;
+            ay[o] = fy;
+            az[o] = fz;
         }
     }
-    // walk statistics: one atomic per warp (every lane of the warp leaves the
-    // walk loop together)
-    for (int o = 16; o > 0; o >>= 1) {
-        visits += __shfl_down_sync(0xffffffffu, visits, o);
-        pairs += __shfl_down_sync(0xffffffffu, pairs, o);
-    }
+    // walk statistics: one atomic per warp, spread over kCounters pairs
+    const unsigned all_visits = __reduce_add_sync(kAll, visits);
+    const unsigned all_pairs = __reduce_add_sync(kAll, pairs);
     if (lane == 0) {
-        atomicAdd(&counters[0], visits);
-        atomicAdd(&counters[1], pairs);
+        unsigned long long* c = counters + 2 * (blockIdx.x % kCounters);
+        atomicAdd(&c[0], static_cast<unsigned long long>(all_visits));
+        atomicAdd(&c[1], static_cast<unsigned long long>(all_pairs));
     }
+}
+
+// Chebyshev interpolation of r_s^3 h over t in [0, t_max] at degree `deg`, in
+// monomials of tau; returns the largest dropped relative error seen on a fine
+// grid (relative to h, in long double).
+long double short_h(long double t) {
+    const long double isp = 0.564189583547756286948079451560772586L;
+    if (t <= 4.0L) {   // the alternating series, terms falling from the first
+        long double term = 1.0L / 4.0L, sum = 0.0L;   // t^k / (4^(k+1) (k+1)!)
+        for (int k = 0; k < 40; ++k) {
+            sum += (k & 1 ? -term : term) * 2.0L * (k + 1) / (2 * k + 3);
+            term *= t / (4.0L * (k + 2));
+        }
+        return isp * sum;
+    }
+    const long double q = std::sqrt(t);
+    return (std::erf(0.5L * q) - q * isp * std::exp(-0.25L * t)) / (t * q);
+}
+
+long double fit_poly(int deg, double t_max, double r_s, PairPoly* out) {
+    const int n = deg + 1;
+    const long double pi = 3.141592653589793238462643383279502884L;
+    std::vector<long double> cheb(n), mono(n, 0.0L), a(n, 0.0L), b(n, 0.0L);
+    std::vector<long double> y(n);
+    for (int k = 0; k < n; ++k)
+        y[k] = short_h(0.5L * t_max * (std::cos(pi * (k + 0.5L) / n) + 1.0L));
+    for (int j = 0; j < n; ++j) {
+        long double s = 0.0L;
+        for (int k = 0; k < n; ++k) s += y[k] * std::cos(pi * j * (k + 0.5L) / n);
+        cheb[j] = s * (j ? 2.0L : 1.0L) / n;
+    }
+    // T_j in monomials by the recurrence T_{j+1} = 2 tau T_j - T_{j-1}
+    a[0] = 1.0L;
+    if (n > 1) b[1] = 1.0L;
+    for (int j = 0; j < n; ++j) {
+        for (int k = 0; k < n; ++k) mono[k] += cheb[j] * a[k];
+        std::vector<long double> c(n, 0.0L);
+        for (int k = 0; k < n; ++k) c[k] = (k ? 2.0L * b[k - 1] : 0.0L) - a[k];
+        a = b;
+        b = c;
+    }
+    const long double rs3 = static_cast<long double>(r_s) * r_s * r_s;
+    out->tau = static_cast<double>(2.0L / (static_cast<long double>(t_max) * r_s * r_s));
+    for (int k = 0; k < n; ++k) out->c[k] = static_cast<double>(mono[k] / rs3);
+    long double worst = 0.0L;
+    for (int i = 0; i <= 400; ++i) {
+        const long double tau = -1.0L + 2.0L * i / 400.0L;
+        long double p = 0.0L;
+        for (int k = deg; k >= 0; --k) p = p * tau + mono[k];
+        const long double h = short_h(0.5L * t_max * (tau + 1.0L));
+        worst = std::max(worst, std::fabs(p - h) / h);
+    }
+    return worst;
 }
 
 // Per-particle masses: node mass and centre of mass summed bottom-up, one
@@ -641,6 +1045,77 @@ uint32_t read_u32(const uint32_t* d, cudaStream_t s) {
     return v;
 }
 
+struct WalkArgs {
+    uint32_t nt;
+    const uint32_t* tslot;
+    const double *sx, *sy, *sz, *sm;
+    const unsigned long long* skey;
+    const Node* nodes;
+    const uint4 *ga, *gm, *gc;
+    uint32_t n_nodes;
+    WalkParams W;
+    const uint32_t* out_idx;
+    int add;
+    double *ax, *ay, *az;
+    unsigned long long* counters;
+    unsigned int* status;
+};
+
+template <typename R, int DEG, int G>
+void launch_walk_as(const WalkArgs& A, const PairPoly& pp, cudaStream_t s) {
+    const unsigned blocks = static_cast<unsigned>((static_cast<uint64_t>(A.nt) + G - 1) / G);
+    k_walk<R, DEG, G><<<blocks, 32, 0, s>>>(A.nt, A.tslot, A.sx, A.sy, A.sz, A.sm, A.skey, A.nodes,
+                                             A.ga, A.gm, A.gc, A.n_nodes, A.W, pp, A.out_idx, A.add,
+                                             A.ax, A.ay, A.az, A.counters, A.status);
+}
+
+template <typename R, int DEG>
+void launch_walk_deg(const WalkArgs& A, const PairPoly& pp, int group, cudaStream_t s) {
+    switch (group) {
+        case 1: launch_walk_as<R, DEG, 1>(A, pp, s); break;
+        case 4: launch_walk_as<R, DEG, 4>(A, pp, s); break;
+        case 8: launch_walk_as<R, DEG, 8>(A, pp, s); break;
+        default: launch_walk_as<R, DEG, 16>(A, pp, s); break;
+    }
+}
+
+// The lowest polynomial degree that reaches the form's accuracy over the cutoff
+// sphere: below the binary64 rounding of the factor itself, or a tenth of the
+// FP32 one. r_cut = 4.5 r_s takes 20 and 12 (1e-17 and 7e-9); from about
+// r_cut = 7 r_s on (binary64) the closed form stays.
+template <typename R>
+void launch_walk(const WalkArgs& A, int group, cudaStream_t s) {
+    PairPoly pp{};
+    const double ratio = A.W.r_cut / A.W.r_s;
+    const double t_max = ratio * ratio * (1.0 + 1e-9);
+    const long double want = sizeof(R) == 8 ? 1e-16L : 1e-8L;
+    if (t_max < 100.0) {
+        if constexpr (sizeof(R) == 4) {
+            if (fit_poly(kDegLow, t_max, A.W.r_s, &pp) < want)
+                return launch_walk_deg<R, kDegLow>(A, pp, group, s);
+        }
+        if (fit_poly(kDegMid, t_max, A.W.r_s, &pp) < want)
+            return launch_walk_deg<R, kDegMid>(A, pp, group, s);
+        if (fit_poly(kDegHigh, t_max, A.W.r_s, &pp) < want)
+            return launch_walk_deg<R, kDegHigh>(A, pp, group, s);
+    }
+    launch_walk_deg<R, 0>(A, pp, group, s);
+}
+
+// Targets a warp takes. A larger group shares the node tests among more targets
+// but has a larger box, so more undecided nodes and rejected pairs, and fewer
+// warps. Measured walk ms at G = 4 / 8 / 16 (clustered sources, every source a
+// target): 30,000: 1.0 / 1.5 / 2.3; 262,144: 6.5 / 4.9 / 6.4; 2.1M: 48 / 36 / 32;
+// 16.8M: 357 / 249 / 191 (one lane per target: 15, 48, 168 and 696). Targets that
+// are a sample of the sources lie further apart: of 2.1M sources, 4,096 targets
+// take 0.7 ms at G = 1 (12 at 4; 48 with one lane per target), 131,072 6.2 (9.8),
+// 524,288 23 at G = 1, 17 at 4, 15 at 8 and 25 at 16 (82).
+int walk_group(uint32_t n, uint32_t nt) {
+    if (nt < n / 8 + 1) return 1;
+    if (nt < 100000) return 4;
+    return nt < 1000000 || nt < n / 2 + 1 ? 8 : 16;
+}
+
 thread_local std::string g_err;
 
 }  // namespace
@@ -754,7 +1229,10 @@ int run(const hyowon_treepm_params& P, uint32_t n, const double* x, const double
             k_moments<<<nb(e - b), kT, 0, s>>>(b, e, sx, sy, sz, sm, nodes);
         }
     }
-    if (node_base) k_open_radius<<<nb(node_base), kT, 0, s>>>(node_base, P.theta, nodes);
+    uint4* ga = mem.get<uint4>(node_base);
+    uint4* gm = mem.get<uint4>(node_base);
+    uint4* gc = mem.get<uint4>(node_base);
+    k_walk_nodes<<<nb(node_base), kT, 0, s>>>(node_base, P.theta, P.box_size, nodes, ga, gm, gc);
     cudaEventRecord(ev.e[1], s);
     const uint32_t* dslots = nullptr;
     const uint32_t* out_idx = nullptr;
@@ -787,26 +1265,24 @@ int run(const hyowon_treepm_params& P, uint32_t n, const double* x, const double
     } else {
         out_idx = sval;   // sorted slot t holds source sval[t]
     }
-    unsigned long long* counters = mem.get<unsigned long long>(2);
-    TCK(cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), s));
+    unsigned long long* counters = mem.get<unsigned long long>(2 * kCounters);
+    TCK(cudaMemsetAsync(counters, 0, 2 * kCounters * sizeof(unsigned long long), s));
     const double G = 6.67430e-11 * (1e10 * 1.98847e30) / (3.085677581491367e22 * 1000.0 * 1000.0);
-    WalkParams W{P.box_size, P.cutoff, P.softening, P.theta, P.split_scale, G, P.particle_mass};
+    const WalkParams W{P.box_size, P.cutoff, P.softening, P.split_scale, G, P.particle_mass};
+    const WalkArgs A{nt, dslots, sx, sy, sz, sm, skey, nodes, ga, gm, gc, node_base, W,
+                     out_idx, host_targets ? 0 : 1, ax, ay, az, counters, status};
+    const int group = walk_group(n, nt);
     cudaEventRecord(ev.e[2], s);
-    const unsigned blocks = static_cast<unsigned>((nt + 127) / 128);
-    const int add = host_targets ? 0 : 1;
-    if (P.precision == HYOWON_FP64)
-        k_walk<double><<<blocks, 128, 0, s>>>(nt, dslots, sx, sy, sz, sm, skey, nodes, node_base, W,
-                                               out_idx, add, ax, ay, az, counters, status);
-    else
-        k_walk<float><<<blocks, 128, 0, s>>>(nt, dslots, sx, sy, sz, sm, skey, nodes, node_base, W,
-                                              out_idx, add, ax, ay, az, counters, status);
+    if (P.precision == HYOWON_FP64) launch_walk<double>(A, group, s);
+    else launch_walk<float>(A, group, s);
     TCK(cudaPeekAtLastError());
     cudaEventRecord(ev.e[3], s);
-    unsigned long long cnt[2] = {0, 0};
+    unsigned long long cnt[2] = {0, 0}, cnt_all[2 * kCounters];
     unsigned int st = 0;
-    TCK(cudaMemcpyAsync(cnt, counters, sizeof(cnt), cudaMemcpyDeviceToHost, s));
+    TCK(cudaMemcpyAsync(cnt_all, counters, sizeof(cnt_all), cudaMemcpyDeviceToHost, s));
     TCK(cudaMemcpyAsync(&st, status, sizeof(st), cudaMemcpyDeviceToHost, s));
     TCK(cudaStreamSynchronize(s));
+    for (unsigned i = 0; i < 2 * kCounters; ++i) cnt[i & 1] += cnt_all[i];
     if (stats) {
         float tb = 0.f, tw = 0.f;
         cudaEventElapsedTime(&tb, ev.e[0], ev.e[1]);

@@ -34,15 +34,17 @@ typedef struct hyowon_treepm_params {
     double softening;      /* Plummer eps */
     double theta;          /* opening angle (> 0) */
     double particle_mass;  /* uniform source mass */
-    int precision;         /* HYOWON_FP64 or HYOWON_FP32_FIXED (FP32 pair and
-                              monopole arithmetic, binary64 positions / tree) */
+    int precision;         /* HYOWON_FP64 or HYOWON_FP32_FIXED (the pair factor to
+                              FP32 accuracy; binary64 positions, tree and sums) */
 } hyowon_treepm_params;
 
 /* Short-range accelerations at n_targets target particles (indices into the
  * n sources; the target itself is excluded) from all n sources, written to
  * ax/ay/az[n_targets]. Positions are host arrays, wrapped to [0, L) on entry.
  * stats (may be NULL) receives {tree nodes, max depth, node visits per target,
- * exact pairs per target, build ms, walk ms}. Returns a hyowon_status code. */
+ * exact pairs per target, build ms, walk ms}; neighbouring targets are walked as
+ * a group, and a node that the group visits counts for each of its targets.
+ * Returns a hyowon_status code. */
 int hyowon_treepm_short_forces(const hyowon_treepm_params* params, uint64_t n,
                                const double* x, const double* y, const double* z,
                                uint64_t n_targets, const uint32_t* targets, double* ax,

@@ -1,0 +1,97 @@
+"""GPU tests of the TreePM walk's group sizes, pair polynomials and periodic images.
+
+The walk groups neighbouring targets (1, 4, 8 or 16 by their number and density)
+and evaluates the pair factor by a polynomial whose degree depends on
+r_cut / r_s (a closed form beyond). Every case here opens every node
+(theta = 1e-6), so the result is direct summation: the oracle's long-double sum,
+to 1e-12 relative RMS in binary64 (700 pairs of a few ulp each) and 1e-5 in the
+FP32 form. With theta = 0.5 the same targets give the same accepted set whatever
+the group, so the results agree to summation order (1e-12, and 1e-6 in FP32).
+"""
+import numpy as np
+import pytest
+
+import hyowon_b200 as hb
+from hyowon_b200.treepm import short_range_forces
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"fp64": 1e-12, "fp32": 1e-5}
+
+
+def rel_rms(got, ref):
+    g, r = np.stack(got), np.stack(ref)
+    return float(np.sqrt(np.sum((g - r) ** 2) / np.sum(r ** 2)))
+
+
+def points(n, L, seed):
+    """Half uniform, half in tight clumps, some across the box edge."""
+    rng = np.random.default_rng(seed)
+    p = rng.uniform(0, L, (3, n))
+    k = n // 2
+    centre = rng.uniform(-0.02 * L, L, (3, max(1, n // 300)))
+    p[:, :k] = centre[:, rng.integers(0, centre.shape[1], k)] + rng.normal(0, 0.01 * L, (3, k))
+    return np.mod(p, L)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("ratio", [2.0, 4.5, 6.4, 7.5, 12.0])
+def test_pair_factor_over_cutoff_ratios(oracle, precision, ratio):
+    """Each polynomial degree and the closed form, against the long-double sum."""
+    L, n = 24.0, 3000
+    x, y, z = points(n, L, 3)
+    r_cut, eps = 5.0, 0.04
+    t = np.arange(0, n, 7, dtype=np.uint32)
+    ref = oracle.short_range_direct(L, x, y, z, 1.5, t, r_cut / ratio, r_cut, eps)
+    got = short_range_forces(L, x, y, z, 1.5, t, r_cut / ratio, r_cut, eps, 1e-6, precision)
+    assert rel_rms(got[:3], ref) <= TOL[precision]
+
+
+@pytest.mark.parametrize("n,nt", [(2, 1), (2, 2), (3, 3), (5, 5), (17, 17), (33, 31), (4097, 4097),
+                                  (4097, 2000), (4097, 511), (120011, 120011), (120011, 70000)])
+def test_groups_are_direct_summation(oracle, n, nt):
+    """Remainders of every group size, and targets denser and sparser than it."""
+    L = 30.0
+    x, y, z = points(n, L, n)
+    rng = np.random.default_rng(n + nt)
+    t = rng.permutation(n)[:nt].astype(np.uint32)
+    check = np.arange(nt) if nt <= 4097 else rng.choice(nt, 500, replace=False)
+    r_cut = 14.0 if n <= 33 else 3.0
+    ref = oracle.short_range_direct(L, x, y, z, 1.0, t[check], r_cut / 4.5, r_cut, 0.03)
+    got = short_range_forces(L, x, y, z, 1.0, t, r_cut / 4.5, r_cut, 0.03, 1e-6)
+    got = [g[check] for g in got[:3]]
+    scale = max(float(np.max(np.abs(r))) for r in ref)
+    if scale == 0.0:     # no pair within the cutoff
+        assert max(float(np.max(np.abs(g))) for g in got) == 0.0
+    else:
+        assert rel_rms(got, ref) <= TOL["fp64"]
+
+
+@pytest.mark.parametrize("theta", [0.3, 0.5, 0.9, 1.6])
+@pytest.mark.parametrize("n,L,r_cut", [(900, 10.0, 4.9), (20000, 40.0, 4.0)])
+def test_groups_accept_the_same_nodes(n, L, r_cut, theta):
+    """Few targets (one a warp) and all of them (groups): cutoff spheres that
+    wrap around the box, opening angles below and above the cube diagonal."""
+    x, y, z = points(n, L, 11)
+    args = (r_cut / 4.5, r_cut, 0.05, theta)
+    every = np.arange(n, dtype=np.uint32)
+    full = short_range_forces(L, x, y, z, 1.0, every, *args)
+    few = np.arange(0, n, 16, dtype=np.uint32)
+    one = short_range_forces(L, x, y, z, 1.0, few, *args)
+    assert rel_rms([f[few] for f in full[:3]], one[:3]) <= TOL["fp64"]
+
+
+def test_largest_group_on_a_handle_equals_single_targets():
+    """More than a million sources of a handle (groups of 16) against a sample
+    walked one target a warp."""
+    n, L = 1000003, 100.0
+    x, y, z = points(n, L, 5)
+    r_s, r_cut, eps = 1.0, 4.5, 0.03
+    few = np.arange(0, n, 1009, dtype=np.uint32)
+    one = short_range_forces(L, x, y, z, 1.0, few, r_s, r_cut, eps, 0.5)
+    with hb.PMSolver(hb.MeshGeometry(L, 32), hb.PMForceMethod.treepm_long_range(r_s)) as s:
+        s.upload(x, y, z, uniform_mass=1.0)
+        full = s.treepm_short_forces(0.5, eps, r_cut)
+    assert abs(full[3]["interactions_per_target"] - one[3]["interactions_per_target"]) \
+        < 0.2 * one[3]["interactions_per_target"]
+    assert rel_rms([f[few] for f in full[:3]], one[:3]) <= TOL["fp64"]
