@@ -291,7 +291,6 @@ void set_input_mass(hyowon_pm_t h, double total, uint32_t n) {
 void release_ic_workspace(hyowon_pm_t h) {
     if (h && h->ic_ws) {
         hyowon::ic::workspace_destroy(h->ic_ws);
-    hyowon::adj::destroy_cache(h->adj);
         h->ic_ws = nullptr;
     }
 }

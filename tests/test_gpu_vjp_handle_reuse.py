@@ -1,0 +1,64 @@
+"""GPU tests of hyowon_pm_vjp on a handle that is used again.
+
+A handle keeps the adjoint's plans and work arrays between calls and gives them
+back before other calls that allocate. Each call must equal the stateless
+hyowon_vjp_1lpt_pm of the same inputs: the two run the same kernels and differ
+only in the order of the deposit's atomics (1e-11 relative in binary64, 2e-3 in
+FP32, the spread of repeated stateless calls times ten).
+"""
+import numpy as np
+import pytest
+
+import hyowon_b200 as hb
+from hyowon_b200 import adjoint, ic
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"fp64": 1e-11, "fp32": 2e-3}
+
+
+def inputs(n, N, seed):
+    rng = np.random.default_rng(seed)
+    return rng.standard_normal(n ** 3), 0.3 * rng.standard_normal(N ** 3)
+
+
+def check(solver, box, n, N, steps, every, precision, seed):
+    noise, target = inputs(n, N, seed)
+    args = (box, n, N, 0.05, steps, precision, every)
+    ref = adjoint.DifferentiablePM(*args).loss_and_grad(noise, target)
+    got = adjoint.DifferentiablePM(*args, solver=solver).loss_and_grad(noise, target)
+    tol = TOL[precision]
+    assert abs(got[0] - ref[0]) <= tol * abs(ref[0])
+    assert np.linalg.norm(got[1] - ref[1]) <= tol * np.linalg.norm(ref[1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("N", [32, 24, 27])
+def test_repeated_calls_equal_stateless_ones(N, precision):
+    """More steps, fewer steps, another lattice, a loss without a gradient; on
+    power-of-two, even and odd meshes (the last leave kept potentials at odd
+    element offsets without padding)."""
+    box = 60.0
+    with hb.PMSolver(hb.MeshGeometry(box, N), hb.PMForceMethod.pure_pm(False), precision) as s:
+        for k, (n, steps, every) in enumerate(((16, 3, 2), (16, 6, 4), (16, 2, 1), (20, 4, 3))):
+            check(s, box, n, N, steps, every, precision, 10 * k + N)
+            noise, target = inputs(n, N, k)
+            d = adjoint.DifferentiablePM(box, n, N, 0.05, steps, precision, every, solver=s)
+            assert np.isfinite(d.loss(noise, target))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_vjp_before_and_after_other_work_of_the_handle(precision):
+    """Generated ICs, a step and a spectrum between two gradients: the step
+    releases the IC work arrays, and the adjoint's engines must outlive that."""
+    box, n, N = 60.0, 16, 32
+    with hb.PMSolver(hb.MeshGeometry(box, N), hb.PMForceMethod.pure_pm(False), precision) as s:
+        check(s, box, n, N, 3, 2, precision, 1)
+        p = ic.ICParams(n, box, 3, 0.05, lpt_order=2)
+        s.generate_ics(p, ic.power_table(p, ic.start_spectrum(0.05)), ic.particle_mass(box, n))
+        f = hb.TimeStepper(0.05, 1.0, 0.3).factors()
+        s.kdk_step(f[0][0], f[1][0], f[2][0])
+        s.power_spectrum(8)
+        check(s, box, n, N, 3, 2, precision, 2)
+        s.kdk_step(f[0][1], f[1][1], f[2][1])
+        check(s, box, n, N, 3, 2, precision, 3)
