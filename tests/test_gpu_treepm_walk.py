@@ -95,3 +95,49 @@ def test_largest_group_on_a_handle_equals_single_targets():
     assert abs(full[3]["interactions_per_target"] - one[3]["interactions_per_target"]) \
         < 0.2 * one[3]["interactions_per_target"]
     assert rel_rms([f[few] for f in full[:3]], one[:3]) <= TOL["fp64"]
+
+
+def tree_size(L, x, y, z):
+    """(nodes, depth) from the definition: level by level, the runs of equal
+    63-bit key prefixes whose parent run holds at least two sources."""
+    def spread(v):
+        v = v.astype(np.uint64)
+        for s, k in ((32, 0x1f00000000ffff), (16, 0x1f0000ff0000ff), (8, 0x100f00f00f00f00f),
+                     (4, 0x10c30c30c30c30c3), (2, 0x1249249249249249)):
+            v = (v | (v << np.uint64(s))) & np.uint64(k)
+        return v
+
+    q = [np.minimum(np.floor(c / L * 2097152.0), 2097151).astype(np.uint64) for c in (x, y, z)]
+    key = np.sort((spread(q[0]) << np.uint64(2)) | (spread(q[1]) << np.uint64(1)) | spread(q[2]))
+    nodes, depth, parent_ok = 0, 0, np.ones(key.size, bool)
+    for level in range(22):
+        prefix = key >> np.uint64(3 * (21 - level))
+        _, first, count = np.unique(prefix, return_index=True, return_counts=True)
+        here = int(np.count_nonzero(parent_ok[first]))
+        if here == 0:
+            break
+        nodes, depth = nodes + here, level
+        parent_ok = np.repeat(count, count) >= 2
+    return nodes, depth
+
+
+@pytest.mark.parametrize("n,copies", [(2, 0), (3, 1), (255, 0), (256, 3), (257, 9), (1025, 40),
+                                      (5000, 700)])
+def test_tree_of_tile_edges_and_coincident_sources(oracle, n, copies):
+    """Tiles of the node sweep around 256 sources; `copies` sources repeat others
+    to the last bit (leaves of several sources at the deepest level) or up to a
+    cell of the deepest levels. Node count and depth from the definition, forces
+    from direct summation."""
+    L, r_cut, eps = 20.0, 6.0, 0.02
+    x, y, z = points(n, L, 100 + n)
+    rng = np.random.default_rng(n)
+    src, dst = rng.integers(0, n, copies), rng.permutation(n)[:copies]
+    x[dst], y[dst], z[dst] = x[src], y[src], z[src]
+    near = dst[::2]
+    x[near] = np.mod(x[near] + L * rng.uniform(-3e-6, 3e-6, near.size), L)
+    every = np.arange(n, dtype=np.uint32)
+    got = short_range_forces(L, x, y, z, 1.0, every, r_cut / 4.5, r_cut, eps, 1e-6)
+    assert (int(got[3]["nodes"]), int(got[3]["depth"])) == tree_size(L, x, y, z)
+    ref = oracle.short_range_direct(L, x, y, z, 1.0, every, r_cut / 4.5, r_cut, eps)
+    scale = max(float(np.max(np.abs(r))) for r in ref)
+    assert max(float(np.max(np.abs(g - r))) for g, r in zip(got[:3], ref)) <= 1e-12 * max(scale, 1e-300)
