@@ -458,6 +458,59 @@ T* dmalloc(size_t count, std::vector<void*>& owned) {
     return static_cast<T*>(p);
 }
 
+// One device block that a run's work arrays are carved from (256-byte aligned),
+// kept between the runs of an engine: some sixty cudaMalloc / cudaFree pairs a
+// call took four fifths of a 128^3 gradient's 55 ms.
+class Arena {
+public:
+    template <typename Layout>
+    size_t count(Layout&& layout) {   // bytes that layout()'s arrays take
+        base_ = nullptr;
+        off_ = 0;
+        layout();
+        return off_;
+    }
+    template <typename Layout>
+    void plan(Layout&& layout) {   // runs layout() twice: to count, then to place
+        count(layout);
+        if (off_ > cap_) {
+            release();
+            ACK(cudaMalloc(&block_, off_));
+            cap_ = off_;
+        }
+        base_ = static_cast<char*>(block_);
+        off_ = 0;
+        layout();
+    }
+    template <typename T>
+    T* take(size_t count) {
+        const size_t at = off_;
+        off_ += ((count ? count : 1) * sizeof(T) + 255) & ~static_cast<size_t>(255);
+        return base_ ? reinterpret_cast<T*>(base_ + at) : nullptr;
+    }
+    size_t capacity() const { return cap_; }
+    void release() {
+        cudaFree(block_);
+        block_ = nullptr;
+        cap_ = 0;
+    }
+    Arena() = default;
+    Arena(const Arena&) = delete;
+    Arena& operator=(const Arena&) = delete;
+    ~Arena() { release(); }
+
+private:
+    void* block_ = nullptr;
+    char* base_ = nullptr;
+    size_t cap_ = 0, off_ = 0;
+};
+
+struct Events {
+    cudaEvent_t e[3] = {};
+    Events() { for (auto& v : e) cudaEventCreate(&v); }
+    ~Events() { for (auto& v : e) cudaEventDestroy(v); }
+};
+
 template <typename R>
 class Engine {
 public:
@@ -547,6 +600,13 @@ public:
     }
     void set_config(const VjpConfig& c) { cfg_ = c; }
 
+    // Gives the work arrays of a run back; the next run takes them again.
+    void trim() {
+        cudaStreamSynchronize(s_);
+        arena_.release();
+        lpt_.release();
+    }
+
     ~Engine() {
         poisson::destroy_plan(plan_);
         if (plans_) {
@@ -631,36 +691,78 @@ public:
              double* delta_out, double* timings) {
         const uint64_t S = cfg_.n_steps;
         const uint64_t k = cfg_.ckpt_every > 0 ? cfg_.ckpt_every : 1;
-        std::vector<void*> tmp;
-        cudaEvent_t e0, e1, e2;
-        cudaEventCreate(&e0);
-        cudaEventCreate(&e1);
-        cudaEventCreate(&e2);
-        // ---- 1LPT ---------------------------------------------------------
-        double* d_noise = dmalloc<double>(n_, tmp);
-        double* tab = dmalloc<double>(3 * cfg_.n_nodes, tmp);
-        double* pd[3];
-        for (int a = 0; a < 3; ++a) pd[a] = dmalloc<double>(n_, tmp);
-        ACK(cudaMemcpy(d_noise, noise, sizeof(double) * n_, cudaMemcpyHostToDevice));
-        ACK(cudaMemcpy(tab, cfg_.ln_k, sizeof(double) * cfg_.n_nodes, cudaMemcpyHostToDevice));
-        ACK(cudaMemcpy(tab + cfg_.n_nodes, cfg_.ln_p, sizeof(double) * cfg_.n_nodes, cudaMemcpyHostToDevice));
-        ACK(cudaMemcpy(tab + 2 * cfg_.n_nodes, cfg_.ln_p_y2, sizeof(double) * cfg_.n_nodes, cudaMemcpyHostToDevice));
-        const char* err = nullptr;
-        const int lrc = lpt_ics_device(static_cast<int>(cfg_.n_side), cfg_.box_size, d_noise, tab,
-                                       tab + cfg_.n_nodes, tab + 2 * cfg_.n_nodes,
-                                       static_cast<int>(cfg_.n_nodes), cfg_.momentum_factor, x_, pd,
-                                       status_, s_, &err);
-        if (lrc) throw Fail{lrc, err ? err : "LPT failed"};
-        for (int a = 0; a < 3; ++a) k_from_double<R><<<nb(n_), kT, 0, s_>>>(n_, pd[a], p_[a]);
-        // ---- forward with checkpoints -------------------------------------
+        Events ev;
+        const cudaEvent_t e0 = ev.e[0], e1 = ev.e[1], e2 = ev.e[2];
+        ACK(cudaMemsetAsync(status_, 0, sizeof(unsigned int), s_));
+        const bool want_grad = grad_out && target;
         const uint64_t n_ckpt = (S + k - 1) / k + 1;
+        // Potentials start on 256-byte boundaries, as cuFFT's vector loads need.
+        const uint64_t phi_stride = (cells_ + 63) / 64 * 64;
+        double *d_noise = nullptr, *tab = nullptr, *d_loss = nullptr, *d_delta = nullptr,
+               *d_target = nullptr, *grad = nullptr;
+        double *pd[3], *lx[3] = {}, *lp[3] = {};
+        R *v[3] = {}, *u[3] = {}, *psi = nullptr, *field = nullptr, *kept_block = nullptr;
         std::vector<double*> cx(3 * n_ckpt);
         std::vector<R*> cp(3 * n_ckpt);
-        for (uint64_t c = 0; c < n_ckpt; ++c)
-            for (int a = 0; a < 3; ++a) {
-                cx[3 * c + a] = dmalloc<double>(n_, tmp);
-                cp[3 * c + a] = dmalloc<R>(n_, tmp);
+        bool keep = false;
+        auto layout = [&] {
+            d_noise = arena_.template take<double>(n_);
+            tab = arena_.template take<double>(3 * cfg_.n_nodes);
+            for (int a = 0; a < 3; ++a) pd[a] = arena_.template take<double>(n_);
+            for (uint64_t c = 0; c < 3 * n_ckpt; ++c) {
+                cx[c] = arena_.template take<double>(n_);
+                cp[c] = arena_.template take<R>(n_);
             }
+            if (want_grad) {
+                for (int a = 0; a < 3; ++a) {
+                    lx[a] = arena_.template take<double>(n_);
+                    lp[a] = arena_.template take<double>(n_);
+                    v[a] = arena_.template take<R>(n_);
+                    u[a] = arena_.template take<R>(cells_);
+                }
+                psi = arena_.template take<R>(cells_);
+                grad = arena_.template take<double>(n_);
+            }
+            d_loss = arena_.template take<double>(1);
+            if (delta_out) d_delta = arena_.template take<double>(cells_);
+            if (target) d_target = arena_.template take<double>(cells_);
+            field = arena_.template take<R>(cells_);
+            if (keep) kept_block = arena_.template take<R>((S + 1) * phi_stride);
+        };
+        // The potential of every forward state (S + 1 meshes) is kept when
+        // device memory allows: the reverse pass then re-derives each state's
+        // force by one gather instead of a deposit and a Green's-function
+        // solve. Particle states stay checkpointed every k steps either way.
+        {
+            const char* lerr = nullptr;
+            const int wrc = lpt_.require(static_cast<int>(cfg_.n_side), s_, &lerr);
+            if (wrc) throw Fail{wrc, lerr ? lerr : "LPT failed"};
+        }
+        if (want_grad) {
+            const size_t rest = arena_.count(layout);
+            size_t free_b = 0, total_b = 0;
+            const size_t need = (S + 1) * phi_stride * sizeof(R);
+            keep = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess
+                && rest <= free_b + arena_.capacity()
+                && need + (size_t(1) << 30) < (free_b + arena_.capacity() - rest) / 2;
+        }
+        arena_.plan(layout);
+        // A block of more than 1/32 of the device's memory is given back.
+        struct GiveBack {
+            Arena& a;
+            cudaStream_t s;
+            ~GiveBack() {
+                size_t free_b = 0, total_b = 0;
+                if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || a.capacity() > total_b / 32) {
+                    cudaStreamSynchronize(s);
+                    a.release();
+                }
+            }
+        } give_back{arena_, s_};
+        std::vector<R*> kept;
+        if (keep)
+            for (uint64_t j = 0; j <= S; ++j) kept.push_back(kept_block + j * phi_stride);
+        auto keep_of = [&](uint64_t j) { return kept.empty() ? nullptr : kept[j]; };
         auto save = [&](uint64_t c) {
             for (int a = 0; a < 3; ++a) {
                 ACK(cudaMemcpyAsync(cx[3 * c + a], x_[a], sizeof(double) * n_, cudaMemcpyDeviceToDevice, s_));
@@ -673,44 +775,21 @@ public:
                 ACK(cudaMemcpyAsync(p_[a], cp[3 * c + a], sizeof(R) * n_, cudaMemcpyDeviceToDevice, s_));
             }
         };
-        // Reverse-pass work arrays are allocated before timing starts.
-        double* lx[3];
-        double* lp[3];
-        R* v[3];
-        R* u[3];
-        R* psi = nullptr;
-        const bool want_grad = grad_out && target;
-        if (want_grad) {
-            for (int a = 0; a < 3; ++a) {
-                lx[a] = dmalloc<double>(n_, tmp);
-                lp[a] = dmalloc<double>(n_, tmp);
-                v[a] = dmalloc<R>(n_, tmp);
-                u[a] = dmalloc<R>(cells_, tmp);
-            }
-            psi = dmalloc<R>(cells_, tmp);
-        }
-        // The potential of every forward state (S + 1 meshes) is kept when
-        // device memory allows: the reverse pass then re-derives each state's
-        // force by one gather instead of a deposit and a Green's-function
-        // solve. Particle states stay checkpointed every k steps either way.
-        std::vector<R*> kept;
-        if (want_grad) {
-            size_t free_b = 0, total_b = 0;
-            const size_t need = (S + 1) * cells_ * sizeof(R);
-            if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && need + (size_t(1) << 30) < free_b / 2) {
-                R* block = dmalloc<R>((S + 1) * cells_, tmp);
-                for (uint64_t j = 0; j <= S; ++j) kept.push_back(block + j * cells_);
-            }
-        }
-        auto keep_of = [&](uint64_t j) { return kept.empty() ? nullptr : kept[j]; };
-        double* d_loss = dmalloc<double>(1, tmp);
-        double* d_delta = delta_out ? dmalloc<double>(cells_, tmp) : nullptr;
-        double* d_target = nullptr;
-        if (target) {
-            d_target = dmalloc<double>(cells_, tmp);
-            ACK(cudaMemcpy(d_target, target, sizeof(double) * cells_, cudaMemcpyHostToDevice));
-        }
-        R* field = dmalloc<R>(cells_, tmp);
+        // ---- 1LPT ---------------------------------------------------------
+        ACK(cudaMemcpyAsync(d_noise, noise, sizeof(double) * n_, cudaMemcpyHostToDevice, s_));
+        ACK(cudaMemcpyAsync(tab, cfg_.ln_k, sizeof(double) * cfg_.n_nodes, cudaMemcpyHostToDevice, s_));
+        ACK(cudaMemcpyAsync(tab + cfg_.n_nodes, cfg_.ln_p, sizeof(double) * cfg_.n_nodes, cudaMemcpyHostToDevice, s_));
+        ACK(cudaMemcpyAsync(tab + 2 * cfg_.n_nodes, cfg_.ln_p_y2, sizeof(double) * cfg_.n_nodes, cudaMemcpyHostToDevice, s_));
+        if (target)
+            ACK(cudaMemcpyAsync(d_target, target, sizeof(double) * cells_, cudaMemcpyHostToDevice, s_));
+        const char* err = nullptr;
+        const int lrc = lpt_ics_device(lpt_, static_cast<int>(cfg_.n_side), cfg_.box_size, d_noise, tab,
+                                       tab + cfg_.n_nodes, tab + 2 * cfg_.n_nodes,
+                                       static_cast<int>(cfg_.n_nodes), cfg_.momentum_factor, x_, pd,
+                                       status_, s_, &err);
+        if (lrc) throw Fail{lrc, err ? err : "LPT failed"};
+        for (int a = 0; a < 3; ++a) k_from_double<R><<<nb(n_), kT, 0, s_>>>(n_, pd[a], p_[a]);
+        // ---- forward with checkpoints -------------------------------------
         // Timed: the KDK forward from the 1LPT state, the loss, and the reverse
         // KDK pass (the 1LPT map and its adjoint, one FFT set each, are setup).
         cudaEventRecord(e0, s_);
@@ -772,8 +851,7 @@ public:
             // ---- 1LPT adjoint: g_d = lx_d + pf lp_d -----------------------------
             k_axpy3<<<nb(n_), kT, 0, s_>>>(n_, cfg_.momentum_factor, lp[0], lp[1], lp[2], lx[0],
                                            lx[1], lx[2]);
-            double* grad = dmalloc<double>(n_, tmp);
-            const int arc = lpt_adjoint_device(static_cast<int>(cfg_.n_side), cfg_.box_size, lx, tab,
+            const int arc = lpt_adjoint_device(lpt_, static_cast<int>(cfg_.n_side), cfg_.box_size, lx, tab,
                                                tab + cfg_.n_nodes, tab + 2 * cfg_.n_nodes,
                                                static_cast<int>(cfg_.n_nodes), grad, s_, &err);
             if (arc) throw Fail{arc, err ? err : "LPT adjoint failed"};
@@ -793,10 +871,6 @@ public:
             timings[2] = static_cast<double>(solves_);
             timings[3] = static_cast<double>(vjps_);
         }
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        cudaEventDestroy(e2);
-        for (void* p : tmp) cudaFree(p);
         if (st) throw Fail{HYOWON_ELOGIC, "a position left the mesh domain"};
     }
 
@@ -826,6 +900,8 @@ private:
     R* acc_[3] = {};
     uint64_t solves_ = 0, vjps_ = 0;
     std::vector<void*> owned_;
+    Arena arena_;       // a run's work arrays
+    LptWork lpt_;
 };
 
 thread_local std::string g_adj_err;
@@ -843,6 +919,12 @@ struct Cache {
 };
 
 void destroy_cache(Cache* c) { delete c; }
+
+void trim_cache(Cache* c) {
+    if (!c) return;
+    if (c->e64) c->e64->trim();
+    if (c->e32) c->e32->trim();
+}
 
 int run_cached(Cache** cache, const VjpConfig& cfg, cudaStream_t s, const double* noise,
                const double* target_delta, double* loss, double* grad_noise,

@@ -12,6 +12,8 @@ namespace hyowon::adj {
 // Adjoint engines (plans and work arrays) a handle keeps between VJP calls.
 struct Cache;
 void destroy_cache(Cache* c);
+// Gives the work arrays of the engines back (they are taken again when used).
+void trim_cache(Cache* c);
 // hyowon_vjp_1lpt_pm on stream s with the engine of *cache (created, or
 // re-created when the geometry changed). Returns a hyowon_status code.
 int run_cached(Cache** cache, const VjpConfig& cfg, cudaStream_t s, const double* noise,

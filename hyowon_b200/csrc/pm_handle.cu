@@ -237,6 +237,7 @@ void free_particles(hyowon_pm_t h) {
 
 int ensure_capacity(hyowon_pm_t h, uint32_t n, bool masses) {
     if (n <= h->cap && (!masses || h->mass[0])) return HYOWON_OK;
+    hyowon::adj::trim_cache(h->adj);
     free_particles(h);
     for (int s = 0; s < 2; ++s) {
         for (int a = 0; a < 3; ++a) {
@@ -1025,6 +1026,7 @@ int hyowon_pm_lpt_ics(hyowon_pm_t h, uint64_t n_side, const double* noise, uint6
                       double momentum_factor, double uniform_mass) {
     release_ic_workspace(h);
     if (!h) return HYOWON_EINVAL;
+    hyowon::adj::trim_cache(h->adj);
     if (n_side < 2 || n_side > 2048 || !noise || n_nodes < 2 || !ln_k || !ln_p || !ln_p_y2)
         return fail(h, HYOWON_EINVAL, "LPT requires n_side in [2,2048], noise and a spline table");
     if (!std::isfinite(uniform_mass) || uniform_mass <= 0.0 || !std::isfinite(momentum_factor))
@@ -1064,7 +1066,8 @@ int hyowon_pm_lpt_ics(hyowon_pm_t h, uint64_t n_side, const double* noise, uint6
     }
     if (rc == HYOWON_OK) {
         cudaMemsetAsync(h->d_status, 0, sizeof(unsigned int), h->stream);
-        const int lrc = lpt_ics_device(N, h->L, d_noise, tab, tab + n_nodes, tab + 2 * n_nodes,
+        LptWork lpt;
+        const int lrc = lpt_ics_device(lpt, N, h->L, d_noise, tab, tab + n_nodes, tab + 2 * n_nodes,
                                        static_cast<int>(n_nodes), momentum_factor, tmp_pos,
                                        tmp_mom, h->d_status, h->stream, &err);
         if (lrc) rc = fail(h, lrc, err ? err : "LPT failed");
@@ -1104,6 +1107,7 @@ int hyowon_pm_lpt_ics(hyowon_pm_t h, uint64_t n_side, const double* noise, uint6
 int hyowon_pm_generate_ics(hyowon_pm_t h, const hyowon_ic_params_t* p, uint64_t n_power,
                            const double* power, double uniform_mass) {
     if (!h) return HYOWON_EINVAL;
+    hyowon::adj::trim_cache(h->adj);
     hyowon::ic::Params r;
     const char* err = nullptr;
     int rc = hyowon::ic::resolve(p, &r, &err);
@@ -1652,6 +1656,7 @@ int hyowon_pm_power_spectrum(hyowon_pm_t h, uint64_t mesh_size, int num_bins,
                              int interlaced, hyowon_pk_bin_t* bins) {
     release_ic_workspace(h);
     if (!h || !bins) return HYOWON_EINVAL;
+    hyowon::adj::trim_cache(h->adj);
     if (!h->has_state) return fail(h, HYOWON_ELOGIC, "no particles uploaded");
     const uint64_t N = mesh_size ? mesh_size : static_cast<uint64_t>(h->N);
     if (N < 2 || N > 4096) return fail(h, HYOWON_EINVAL, "MatterPowerSpectrum mesh_size must be in [2, 4096]");

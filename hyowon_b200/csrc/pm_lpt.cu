@@ -158,160 +158,134 @@ __global__ void k_scale(uint64_t n, const double* __restrict__ in, double s, dou
 
 }  // namespace
 
-int lpt_adjoint_device(int N, double L, double* const d_g[3], const double* d_xs,
+static_assert(sizeof(cufftHandle) == sizeof(int), "LptWork keeps plan handles as int");
+
+int LptWork::require(int n_side, cudaStream_t s, const char** err) {
+    *err = nullptr;
+    if (N != n_side || !plans) {
+        release();
+        const size_t cells = static_cast<size_t>(n_side) * n_side * n_side;
+        const size_t half = static_cast<size_t>(n_side) * n_side * (n_side / 2 + 1);
+        size_t w1 = 0, w2 = 0;
+        if (cudaMalloc(&delta, sizeof(double2) * half) != cudaSuccess
+            || cudaMalloc(&work, sizeof(double2) * half) != cudaSuccess
+            || cudaMalloc(&real, sizeof(double) * cells) != cudaSuccess) {
+            *err = "LPT work arrays could not be allocated";
+            release();
+            return 7;
+        }
+        if (cufftCreate(&r2c) != CUFFT_SUCCESS) {
+            *err = "cufftCreate failed";
+            release();
+            return 6;
+        }
+        if (cufftCreate(&c2r) != CUFFT_SUCCESS) {
+            cufftDestroy(r2c);
+            *err = "cufftCreate failed";
+            release();
+            return 6;
+        }
+        plans = true;
+        cufftSetAutoAllocation(r2c, 0);
+        cufftSetAutoAllocation(c2r, 0);
+        if (cufftMakePlan3d(r2c, n_side, n_side, n_side, CUFFT_D2Z, &w1) != CUFFT_SUCCESS
+            || cufftMakePlan3d(c2r, n_side, n_side, n_side, CUFFT_Z2D, &w2) != CUFFT_SUCCESS) {
+            *err = "cuFFT plan for the IC mesh failed";
+            release();
+            return 6;
+        }
+        if (cudaMalloc(&fft, w1 > w2 ? w1 : w2) != cudaSuccess) {
+            *err = "cuFFT workspace could not be allocated";
+            release();
+            return 7;
+        }
+        cufftSetWorkArea(r2c, fft);
+        cufftSetWorkArea(c2r, fft);
+        N = n_side;
+    }
+    cufftSetStream(r2c, s);
+    cufftSetStream(c2r, s);
+    return 0;
+}
+
+void LptWork::release() {
+    if (plans) {
+        cufftDestroy(r2c);
+        cufftDestroy(c2r);
+    }
+    plans = false;
+    cudaFree(fft);
+    cudaFree(delta);
+    cudaFree(work);
+    cudaFree(real);
+    fft = nullptr;
+    delta = work = nullptr;
+    real = nullptr;
+    N = 0;
+}
+
+int lpt_adjoint_device(LptWork& w, int N, double L, double* const d_g[3], const double* d_xs,
                        const double* d_ys, const double* d_y2, int n_nodes, double* d_grad,
                        cudaStream_t s, const char** err) {
     const size_t cells = static_cast<size_t>(N) * N * N;
     const size_t half = static_cast<size_t>(N) * N * (N / 2 + 1);
-    double2* gk = nullptr;
-    double2* acc = nullptr;
-    double* real = nullptr;
-    void* ws = nullptr;
-    cufftHandle r2c = 0, c2r = 0;
-    bool hr = false, hc = false;
-    size_t w1 = 0, w2 = 0;
-    int rc = 0;
-    *err = nullptr;
+    if (const int rc = w.require(N, s, err)) return rc;
     const unsigned bh = static_cast<unsigned>((half + 255) / 256);
     const unsigned bc = static_cast<unsigned>((cells + 255) / 256);
     const double norm = static_cast<double>(cells) / (L * L * L);
-    if (cudaMalloc(&gk, sizeof(double2) * half) != cudaSuccess
-        || cudaMalloc(&acc, sizeof(double2) * half) != cudaSuccess
-        || cudaMalloc(&real, sizeof(double) * cells) != cudaSuccess) {
-        *err = "LPT adjoint work arrays could not be allocated";
-        rc = 7;
-        goto done;
-    }
-    if (cufftCreate(&r2c) != CUFFT_SUCCESS || cufftCreate(&c2r) != CUFFT_SUCCESS) {
-        *err = "cufftCreate failed";
-        rc = 6;
-        goto done;
-    }
-    hr = hc = true;
-    cufftSetAutoAllocation(r2c, 0);
-    cufftSetAutoAllocation(c2r, 0);
-    if (cufftMakePlan3d(r2c, N, N, N, CUFFT_D2Z, &w1) != CUFFT_SUCCESS
-        || cufftMakePlan3d(c2r, N, N, N, CUFFT_Z2D, &w2) != CUFFT_SUCCESS
-        || cudaMalloc(&ws, w1 > w2 ? w1 : w2) != cudaSuccess) {
-        *err = "cuFFT plan for the LPT adjoint failed";
-        rc = 6;
-        goto done;
-    }
-    cufftSetWorkArea(r2c, ws);
-    cufftSetWorkArea(c2r, ws);
-    cufftSetStream(r2c, s);
-    cufftSetStream(c2r, s);
     for (int a = 0; a < 3; ++a) {
         // the D2Z input is copied so the caller's cotangent survives
-        cudaMemcpyAsync(real, d_g[a], sizeof(double) * cells, cudaMemcpyDeviceToDevice, s);
-        if (cufftExecD2Z(r2c, real, reinterpret_cast<cufftDoubleComplex*>(gk)) != CUFFT_SUCCESS) {
+        cudaMemcpyAsync(w.real, d_g[a], sizeof(double) * cells, cudaMemcpyDeviceToDevice, s);
+        if (cufftExecD2Z(w.r2c, w.real, reinterpret_cast<cufftDoubleComplex*>(w.work)) != CUFFT_SUCCESS) {
             *err = "LPT adjoint r2c failed";
-            rc = 6;
-            goto done;
+            return 6;
         }
-        k_lpt_adjoint_accumulate<<<bh, 256, 0, s>>>(N, L, a, gk, d_xs, d_ys, d_y2, n_nodes, norm,
-                                                    a == 0, acc);
+        k_lpt_adjoint_accumulate<<<bh, 256, 0, s>>>(N, L, a, w.work, d_xs, d_ys, d_y2, n_nodes, norm,
+                                                    a == 0, w.delta);
     }
-    if (cufftExecZ2D(c2r, reinterpret_cast<cufftDoubleComplex*>(acc), real) != CUFFT_SUCCESS) {
+    if (cufftExecZ2D(w.c2r, reinterpret_cast<cufftDoubleComplex*>(w.delta), w.real) != CUFFT_SUCCESS) {
         *err = "LPT adjoint c2r failed";
-        rc = 6;
-        goto done;
+        return 6;
     }
     // grad = -(1/N^3) c2r(acc): the displacement operator is antisymmetric.
-    k_scale<<<bc, 256, 0, s>>>(cells, real, -1.0 / static_cast<double>(cells), d_grad);
+    k_scale<<<bc, 256, 0, s>>>(cells, w.real, -1.0 / static_cast<double>(cells), d_grad);
     if (cudaStreamSynchronize(s) != cudaSuccess) {
         *err = "LPT adjoint kernels failed";
-        rc = 6;
+        return 6;
     }
-done:
-    if (hr) cufftDestroy(r2c);
-    if (hc) cufftDestroy(c2r);
-    cudaFree(ws);
-    cudaFree(gk);
-    cudaFree(acc);
-    cudaFree(real);
-    return rc;
+    return 0;
 }
 
-int lpt_ics_device(int N, double L, const double* d_noise, const double* d_xs,
+int lpt_ics_device(LptWork& w, int N, double L, const double* d_noise, const double* d_xs,
                    const double* d_ys, const double* d_y2, int n_nodes, double pf,
                    double* const d_pos[3], double* const d_mom[3], unsigned int* d_status,
                    cudaStream_t s, const char** err) {
     const size_t cells = static_cast<size_t>(N) * N * N;
     const size_t half = static_cast<size_t>(N) * N * (N / 2 + 1);
-    double2* delta = nullptr;
-    double2* work = nullptr;
-    double* real = nullptr;
-    void* fft_ws = nullptr;
-    cufftHandle r2c = 0, c2r = 0;
-    bool have_r2c = false, have_c2r = false;
-    int rc = 0;
-    size_t ws1 = 0, ws2 = 0;
-    *err = nullptr;
-    if (cudaMalloc(&delta, sizeof(double2) * half) != cudaSuccess
-        || cudaMalloc(&work, sizeof(double2) * half) != cudaSuccess
-        || cudaMalloc(&real, sizeof(double) * cells) != cudaSuccess) {
-        *err = "LPT work arrays could not be allocated";
-        rc = 7;
-        goto done;
+    if (const int rc = w.require(N, s, err)) return rc;
+    const unsigned bh = static_cast<unsigned>((half + 255) / 256);
+    const unsigned bc = static_cast<unsigned>((cells + 255) / 256);
+    const double norm = static_cast<double>(cells) / (L * L * L);
+    const double inv_n3 = 1.0 / (static_cast<double>(N) * N * N);
+    if (cufftExecD2Z(w.r2c, const_cast<double*>(d_noise),
+                     reinterpret_cast<cufftDoubleComplex*>(w.delta)) != CUFFT_SUCCESS) {
+        *err = "IC r2c failed";
+        return 6;
     }
-    if (cufftCreate(&r2c) != CUFFT_SUCCESS || cufftCreate(&c2r) != CUFFT_SUCCESS) {
-        *err = "cufftCreate failed";
-        rc = 6;
-        goto done;
-    }
-    have_r2c = have_c2r = true;
-    cufftSetAutoAllocation(r2c, 0);
-    cufftSetAutoAllocation(c2r, 0);
-    if (cufftMakePlan3d(r2c, N, N, N, CUFFT_D2Z, &ws1) != CUFFT_SUCCESS
-        || cufftMakePlan3d(c2r, N, N, N, CUFFT_Z2D, &ws2) != CUFFT_SUCCESS) {
-        *err = "cuFFT plan for the IC mesh failed";
-        rc = 6;
-        goto done;
-    }
-    if (cudaMalloc(&fft_ws, ws1 > ws2 ? ws1 : ws2) != cudaSuccess) {
-        *err = "cuFFT workspace could not be allocated";
-        rc = 7;
-        goto done;
-    }
-    cufftSetWorkArea(r2c, fft_ws);
-    cufftSetWorkArea(c2r, fft_ws);
-    cufftSetStream(r2c, s);
-    cufftSetStream(c2r, s);
-    {
-        const unsigned bh = static_cast<unsigned>((half + 255) / 256);
-        const unsigned bc = static_cast<unsigned>((cells + 255) / 256);
-        const double norm = static_cast<double>(cells) / (L * L * L);
-        const double inv_n3 = 1.0 / (static_cast<double>(N) * N * N);
-        if (cufftExecD2Z(r2c, const_cast<double*>(d_noise),
-                         reinterpret_cast<cufftDoubleComplex*>(delta)) != CUFFT_SUCCESS) {
-            *err = "IC r2c failed";
-            rc = 6;
-            goto done;
+    k_lpt_amplitude<<<bh, 256, 0, s>>>(N, L, w.delta, d_xs, d_ys, d_y2, n_nodes, norm, d_status);
+    for (int a = 0; a < 3; ++a) {
+        k_lpt_psi<<<bh, 256, 0, s>>>(N, L, a, w.delta, w.work);
+        if (cufftExecZ2D(w.c2r, reinterpret_cast<cufftDoubleComplex*>(w.work), w.real) != CUFFT_SUCCESS) {
+            *err = "IC c2r failed";
+            return 6;
         }
-        k_lpt_amplitude<<<bh, 256, 0, s>>>(N, L, delta, d_xs, d_ys, d_y2, n_nodes, norm, d_status);
-        for (int a = 0; a < 3; ++a) {
-            k_lpt_psi<<<bh, 256, 0, s>>>(N, L, a, delta, work);
-            if (cufftExecZ2D(c2r, reinterpret_cast<cufftDoubleComplex*>(work), real) != CUFFT_SUCCESS) {
-                *err = "IC c2r failed";
-                rc = 6;
-                goto done;
-            }
-            k_lpt_apply<<<bc, 256, 0, s>>>(N, L, a, real, inv_n3, pf, d_pos[a], d_mom[a]);
-        }
-        if (cudaStreamSynchronize(s) != cudaSuccess) {
-            *err = "LPT kernels failed";
-            rc = 6;
-        }
+        k_lpt_apply<<<bc, 256, 0, s>>>(N, L, a, w.real, inv_n3, pf, d_pos[a], d_mom[a]);
     }
-done:
-    if (have_r2c) cufftDestroy(r2c);
-    if (have_c2r) cufftDestroy(c2r);
-    cudaFree(fft_ws);
-    cudaFree(delta);
-    cudaFree(work);
-    cudaFree(real);
-    return rc;
+    if (cudaStreamSynchronize(s) != cudaSuccess) {
+        *err = "LPT kernels failed";
+        return 6;
+    }
+    return 0;
 }
 
 }  // namespace hyowon
