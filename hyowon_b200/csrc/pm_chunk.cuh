@@ -22,6 +22,16 @@
 #endif
 
 namespace hyowon {
+
+// Rows of a deposit tile: `cells` cells, at least one row and at most N, fewer
+// (a power of two) where that would leave fewer than 320 tiles, two for each SM.
+__host__ __device__ constexpr int deposit_tile_rows(int N, int cells) {
+    int rows = cells / N < 1 ? 1 : (cells / N > N ? N : cells / N);
+    int fill = 1;
+    while (2 * fill * 320 <= N * N) fill *= 2;
+    return rows > fill ? fill : rows;
+}
+
 namespace chunked {
 
 using fft::cx_t;

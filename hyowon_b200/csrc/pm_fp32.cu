@@ -188,20 +188,13 @@ k_kick_drift_key(uint32_t n, const uint32_t* __restrict__ ux,
     block_max_to(static_cast<unsigned long long>(__double_as_longlong(drift_max)), max_drift_bits);
 }
 
-__global__ void k_max_count(uint32_t nb, const uint32_t* __restrict__ count, uint32_t* max_count) {
-    uint32_t m = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += gridDim.x * blockDim.x)
-        m = max(m, count[i]);
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(max_count, m);
-}
-
 // Chooses the deposit fraction bits B for this step: the largest B <= 16 with
 // 8 * max_bucket * 2^(3B) <= 2^63 - 1, so no cell (fed by at most 8 buckets'
 // particles) can overflow; then the mean offset and the Green constant.
 __global__ void k_plan(uint32_t n, uint64_t cells, const uint32_t* max_count, double c0,
-                       int centre, FixedPlan* plan) {
+                       int centre, FixedPlan* plan, unsigned long long* qsum) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    if (qsum) *qsum = 0ull;   // the deposit sums into it
     const unsigned long long mc = *max_count > 0 ? *max_count : 1u;
     int B = 16;
     while (B > 4) {
@@ -272,8 +265,7 @@ __device__ __forceinline__ void shared_add_u64(unsigned long long* a, unsigned l
 #define HYOWON_DEPOSIT_TILE_CELLS 4096
 #endif
 __host__ __device__ constexpr int deposit_rows(int N) {
-    return HYOWON_DEPOSIT_TILE_CELLS / N < 1 ? 1
-         : (HYOWON_DEPOSIT_TILE_CELLS / N > N ? N : HYOWON_DEPOSIT_TILE_CELLS / N);
+    return deposit_tile_rows(N, HYOWON_DEPOSIT_TILE_CELLS);
 }
 
 #ifndef HYOWON_DEPOSIT_MINB
@@ -564,8 +556,11 @@ k_gather_kick(uint32_t n, const float* __restrict__ phi, const uint32_t* __restr
               const float* __restrict__ pz, float* __restrict__ ax, float* __restrict__ ay,
               float* __restrict__ az, int do_kick, float K2, float* __restrict__ pxo,
               float* __restrict__ pyo, float* __restrict__ pzo, int N, float inv_two_dx,
-              unsigned int* status) {
+              unsigned int* status, const unsigned long long* qsum, const FixedPlan* plan,
+              unsigned long long expect_offset) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    // the exact mesh-sum identity of the deposit (k_check_mass), one thread
+    if (i == 0 && *qsum != plan->residual + expect_offset) raise_status(status, ST_MASS);
     if (i >= n || (*status & ST_BLOCKS_PUBLISH)) return;
     // the momenta load while the stencil does (2.96 -> 2.60 ms at 512^3 / 1024^3;
     // the binary64 gather, at 48 registers with spills, was slower so)
@@ -701,7 +696,7 @@ struct State {
     double input_mass = 0.0;
     SortWork sort{};
     uint32_t sort_cap = 0;
-    uint32_t* d_max_count = nullptr;
+    uint32_t* d_max_count = nullptr;   // the handle's
     FixedPlan* d_plan = nullptr;
     unsigned long long* d_qsum = nullptr;
     uint32_t* order = nullptr;   // cell order of unmoved particles (steps between re-sorts)
@@ -833,8 +828,10 @@ double green_c0(const State* st) {
 }  // namespace
 
 int create(State** out, double L, int N, int method, int deconvolve, double r_s,
-           const double* lap, const double* win, double four_pi_G, cudaStream_t s) {
+           const double* lap, const double* win, double four_pi_G, uint32_t* max_count,
+           cudaStream_t s) {
     State* st = new State();
+    st->d_max_count = max_count;
     *out = st;
     st->L = L;
     st->N = N;
@@ -858,7 +855,6 @@ int create(State** out, double L, int N, int method, int deconvolve, double r_s,
     if (method == HYOWON_TREEPM_LONG_RANGE) CK(dalloc(&st->phi_k, half));
     CK(dalloc(&st->lap, N));
     CK(dalloc(&st->win, N));
-    CK(dalloc(&st->d_max_count, 1));
     CK(dalloc(&st->d_plan, 1));
     CK(dalloc(&st->d_qsum, 1));
     std::vector<float> lf(N), wf(N);
@@ -914,7 +910,6 @@ void destroy(State* st) {
     cudaFree(st->phi_k);
     cudaFree(st->lap);
     cudaFree(st->win);
-    cudaFree(st->d_max_count);
     cudaFree(st->d_plan);
     cudaFree(st->d_qsum);
     cudaFree(st->d_flag);
@@ -1009,11 +1004,8 @@ int sort_current(State* st, cudaStream_t s, unsigned int* d_status) {
     k_key<<<blocks_for(n), kThreads, 0, s>>>(n, st->pos[st->pc][0], st->pos[st->pc][1],
                                              st->pos[st->pc][2], st->N, st->sort.shift, st->sort.key,
                                              st->sort.rank, st->sort.count, st->d_max_count);
-    ++st->launches;
-    k_max_count<<<st->fill_blocks, kThreads, 0, s>>>(st->sort.n_buckets, st->sort.count,
-                                                     st->d_max_count);
     st->launches += launch_exclusive_scan(st->sort.count, st->sort.offset, st->sort.n_buckets + 1,
-                          st->sort.scan_tmp, s);
+                                          st->sort.scan_tmp, s, st->d_max_count);
     const uint32_t* src[7];
     uint32_t* dst[7];
     for (int a = 0; a < 3; ++a) {
@@ -1101,13 +1093,15 @@ int enqueue_force_sets(State* st, cudaStream_t s, unsigned int* d_status, bool k
     const uint64_t half = static_cast<uint64_t>(N) * N * (N / 2 + 1);
     rec(ev, 1, s);
     ++st->launches;
-    k_plan<<<1, 32, 0, s>>>(n, cells, st->d_max_count, green_c0(st), 1, st->d_plan);
-    CK(cudaMemsetAsync(st->d_qsum, 0, sizeof(unsigned long long), s));
+    k_plan<<<1, 32, 0, s>>>(n, cells, st->d_max_count, green_c0(st), 1, st->d_plan,
+                            st->d_qsum);
     int rc = st->five_pass ? deposit_spectrum(st, P, order, st->d_qsum, d_status, s)
                            : deposit_tiles<float>(st, P, order, st->rmesh, st->d_qsum, d_status, s);
     if (rc) return rc;
-    ++st->launches;
-    k_check_mass<<<1, 32, 0, s>>>(st->d_qsum, st->d_plan, st->mass_check_offset, d_status);
+    if (st->method != HYOWON_PURE_PM) {   // else the gather checks it
+        ++st->launches;
+        k_check_mass<<<1, 32, 0, s>>>(st->d_qsum, st->d_plan, st->mass_check_offset, d_status);
+    }
     float* const pxo = st->mom[1 - M][0];
     float* const pyo = st->mom[1 - M][1];
     float* const pzo = st->mom[1 - M][2];
@@ -1135,12 +1129,14 @@ int enqueue_force_sets(State* st, cudaStream_t s, unsigned int* d_status, bool k
             k_gather_kick<uint32_t><<<blocks_for(n), kThreads, 0, s>>>(
                 n, st->rmesh, st->pos[P][0], st->pos[P][1], st->pos[P][2],
                 st->mom[M][0], st->mom[M][1], st->mom[M][2], st->acc[0], st->acc[1],
-                st->acc[2], kick ? 1 : 0, K2f, pxo, pyo, pzo, N, inv_two_dx, d_status);
+                st->acc[2], kick ? 1 : 0, K2f, pxo, pyo, pzo, N, inv_two_dx, d_status,
+                st->d_qsum, st->d_plan, st->mass_check_offset);
         else
             k_gather_kick<uint64_t><<<blocks_for(n), kThreads, 0, s>>>(
                 n, st->rmesh, st->pos[P][0], st->pos[P][1], st->pos[P][2],
                 st->mom[M][0], st->mom[M][1], st->mom[M][2], st->acc[0], st->acc[1],
-                st->acc[2], kick ? 1 : 0, K2f, pxo, pyo, pzo, N, inv_two_dx, d_status);
+                st->acc[2], kick ? 1 : 0, K2f, pxo, pyo, pzo, N, inv_two_dx, d_status,
+                st->d_qsum, st->d_plan, st->mass_check_offset);
         rec(ev, 6, s);
         return HYOWON_OK;
     }
@@ -1160,12 +1156,14 @@ int enqueue_force_sets(State* st, cudaStream_t s, unsigned int* d_status, bool k
             k_gather_kick<uint32_t><<<blocks_for(n), kThreads, 0, s>>>(
                 n, st->rmesh, st->pos[P][0], st->pos[P][1], st->pos[P][2],
                 st->mom[M][0], st->mom[M][1], st->mom[M][2], st->acc[0], st->acc[1],
-                st->acc[2], kick ? 1 : 0, K2f, pxo, pyo, pzo, N, inv_two_dx, d_status);
+                st->acc[2], kick ? 1 : 0, K2f, pxo, pyo, pzo, N, inv_two_dx, d_status,
+                st->d_qsum, st->d_plan, st->mass_check_offset);
         else
             k_gather_kick<uint64_t><<<blocks_for(n), kThreads, 0, s>>>(
                 n, st->rmesh, st->pos[P][0], st->pos[P][1], st->pos[P][2],
                 st->mom[M][0], st->mom[M][1], st->mom[M][2], st->acc[0], st->acc[1],
-                st->acc[2], kick ? 1 : 0, K2f, pxo, pyo, pzo, N, inv_two_dx, d_status);
+                st->acc[2], kick ? 1 : 0, K2f, pxo, pyo, pzo, N, inv_two_dx, d_status,
+                st->d_qsum, st->d_plan, st->mass_check_offset);
         rec(ev, 6, s);
         return HYOWON_OK;
     }
@@ -1204,10 +1202,8 @@ int kdk_step(State* st, cudaStream_t s, unsigned int* d_status, unsigned long lo
              double K1, double D, double K2, cudaEvent_t* ev) {
     const uint32_t n = st->n;
     const bool sort_now = st->sort_interval <= 1 || st->since_sort + 1 >= st->sort_interval;
-    CK(cudaMemsetAsync(d_status, 0, sizeof(unsigned int), s));
-    CK(cudaMemsetAsync(d_maxdrift, 0, sizeof(unsigned long long), s));
+    // the caller has zeroed the status, the drift maximum and the largest count
     CK(cudaMemsetAsync(st->sort.count, 0, sizeof(uint32_t) * (st->sort.n_buckets + 1), s));
-    CK(cudaMemsetAsync(st->d_max_count, 0, sizeof(uint32_t), s));
     rec(ev, 0, s);
     const int pc = st->pc, mc = st->mc;
     ++st->launches;
@@ -1223,7 +1219,7 @@ int kdk_step(State* st, cudaStream_t s, unsigned int* d_status, unsigned long lo
     // cell order of the candidate positions: bucket offsets every step; the
     // particle arrays themselves are permuted only on re-sort steps
     st->launches += launch_exclusive_scan(st->sort.count, st->sort.offset, st->sort.n_buckets + 1,
-                                          st->sort.scan_tmp, s);
+                                          st->sort.scan_tmp, s, st->d_max_count);
     st->step_perm = !sort_now;
     if (!sort_now) {
         ++st->launches;
@@ -1247,9 +1243,6 @@ int kdk_step(State* st, cudaStream_t s, unsigned int* d_status, unsigned long lo
         P = pc;
         M = mc;
     }
-    ++st->launches;
-    k_max_count<<<st->fill_blocks, kThreads, 0, s>>>(st->sort.n_buckets, st->sort.count,
-                                                     st->d_max_count);
     st->step_P = P;
     st->step_M = M;
     return enqueue_force_sets(st, s, d_status, true, K2, ev, P, M,
@@ -1438,7 +1431,7 @@ int download_mass_mesh(State* st, cudaStream_t s, unsigned int* d_status, double
         if (rc) return rc;
     }
     ++st->launches;
-    k_plan<<<1, 32, 0, s>>>(n, cells, st->d_max_count, green_c0(st), 0, st->d_plan);
+    k_plan<<<1, 32, 0, s>>>(n, cells, st->d_max_count, green_c0(st), 0, st->d_plan, nullptr);
     CK(cudaMemsetAsync(d_status, 0, sizeof(unsigned int), s));
     long long* q = nullptr;
     CK(dalloc(&q, cells));

@@ -30,7 +30,8 @@ struct State;
 using ShortRangeHook = int (*)(void* ctx, cudaStream_t s, int position_set);
 
 int create(State** out, double L, int N, int method, int deconvolve, double r_s,
-           const double* lap, const double* win, double four_pi_G, cudaStream_t s);
+           const double* lap, const double* win, double four_pi_G, uint32_t* max_count,
+           cudaStream_t s);
 void destroy(State* st);
 const std::string& last_error(State* st);
 

@@ -238,8 +238,7 @@ constexpr int kDepositBatch = HYOWON_DEPOSIT64_BATCH;
 // Tile rows for 8-byte-per-cell accumulators of HYOWON_DEPOSIT64_TILE_CELLS
 // cells, halved for the two-word form (same shared memory per tile).
 __host__ __device__ constexpr int tile_rows_f64(int N, int words) {
-    return HYOWON_DEPOSIT64_TILE_CELLS / words / N < 1 ? 1
-         : (HYOWON_DEPOSIT64_TILE_CELLS / words / N > N ? N : HYOWON_DEPOSIT64_TILE_CELLS / words / N);
+    return deposit_tile_rows(N, HYOWON_DEPOSIT64_TILE_CELLS / words);
 }
 
 __device__ __forceinline__ int fixed_split_bits(const uint32_t* max_count) {
@@ -432,15 +431,6 @@ k_deposit_tiles(const double* __restrict__ x, const double* __restrict__ y,
         for (int e = tid; e < tcells; e += kTileThreads)
             out[e] = fixed_to_double(acc_hi[e], acc_lo[e], W) * from_fixed;
     }
-}
-
-__global__ void k_max_count64(uint32_t nb, const uint32_t* __restrict__ count,
-                              uint32_t* max_count) {
-    uint32_t m = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += gridDim.x * blockDim.x)
-        m = max(m, count[i]);
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(max_count, m);
 }
 
 // Pure-PM Green's function (src/mesh/green_function.cpp:165-207) applied to the
@@ -913,11 +903,18 @@ cudaError_t launch_tiles_n(const ParticlesF64& p, const double* mass, double uni
 cudaError_t launch_deposit_tiles_f64(const ParticlesF64& p, const double* mass,
                                      double uniform_mass, const uint32_t* order,
                                      const SortWork& w, Axis a, const uint32_t* max_count,
-                                     uint32_t max_count_host, int e_max, double* mesh,
+                                     const uint32_t* max_count_host, int e_max, double* mesh,
                                      double2* modes, const double2* tw, unsigned int* status,
                                      cudaStream_t s) {
     // the same W the kernels derive from *max_count (they check it again)
-    const unsigned long long c = 8ull * (max_count_host > 0u ? max_count_host : 1u);
+    if (!max_count_host) {
+        const cudaError_t e = launch_tiles_n<1>(p, mass, uniform_mass, order, w, a, max_count, e_max,
+                                                mesh, modes, tw, status, s);
+        if (e != cudaSuccess) return e;
+        return launch_tiles_n<2>(p, mass, uniform_mass, order, w, a, max_count, e_max, mesh, modes,
+                                 tw, status, s);
+    }
+    const unsigned long long c = 8ull * (*max_count_host > 0u ? *max_count_host : 1u);
     int lg = 0;
     while ((c >> (lg + 1)) != 0ull) ++lg;
     const int W = 63 - lg;
@@ -927,14 +924,6 @@ cudaError_t launch_deposit_tiles_f64(const ParticlesF64& p, const double* mass,
     return launch_tiles_n<2>(p, mass, uniform_mass, order, w, a, max_count, e_max, mesh, modes, tw,
                              status, s);
 }
-
-void launch_max_count_f64(uint32_t n_buckets, const uint32_t* count, uint32_t* max_count,
-                          cudaStream_t s) {
-    k_max_count64<<<stream_blocks(n_buckets, kThreads), kThreads, 0, s>>>(n_buckets, count,
-                                                                          max_count);
-}
-
-
 
 void launch_green_f64(int N, double2* modes, const double* lap, const double* win,
                       double four_pi_G, double scale, int deconvolve, double input_mass,

@@ -60,6 +60,13 @@ struct Error {
     std::string msg;
 };
 
+// What a step reports to the host, zeroed and read back in one piece.
+struct StepWords {
+    unsigned int status;            // StatusBits
+    uint32_t max_count;             // largest bucket count of the last keying
+    unsigned long long max_drift;   // bits of the largest drift
+};
+
 }  // namespace
 
 struct hyowon_pm_s {
@@ -111,18 +118,17 @@ struct hyowon_pm_s {
     SortWork sort{};
     uint32_t sort_cap_buckets = 0;
     uint32_t* order = nullptr;        // cell-order slot -> particle slot (n)
-    uint32_t* d_max_count = nullptr;  // largest bucket count of the last keying
     double max_mass = 0.0;            // largest particle mass (fixed-point scale)
     // What the bucket offsets describe for the current position set:
     // 0 nothing, 1 the arrays themselves are in cell order, 2 `order` holds it.
     int order_state = 0;
 
-    unsigned int* d_status = nullptr;
+    StepWords* d_words = nullptr;
+    unsigned int* d_status = nullptr;           // members of *d_words
+    uint32_t* d_max_count = nullptr;
     unsigned long long* d_maxdrift = nullptr;
     double* d_diag = nullptr;                   // diagnostics scratch (pm_diag.h)
-    unsigned int* h_status = nullptr;           // pinned
-    uint32_t* h_max_count = nullptr;            // pinned
-    unsigned long long* h_maxdrift = nullptr;   // pinned
+    StepWords* h_words = nullptr;               // pinned
 
     fp32::State* f32 = nullptr;  // precision form (pm_fp32.cu)
 
@@ -297,21 +303,26 @@ void release_ic_workspace(hyowon_pm_t h) {
 }
 
 int read_status(hyowon_pm_t h, unsigned int* st) {
-    CK(cudaMemcpyAsync(h->h_status, h->d_status, sizeof(unsigned int), cudaMemcpyDeviceToHost,
-                       h->stream));
+    CK(cudaMemcpyAsync(h->h_words, h->d_words, sizeof(StepWords), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    *st = *h->h_status;
+    *st = h->h_words->status;
     return HYOWON_OK;
+}
+
+// The largest drift of the step whose status was just read.
+double drift_read(hyowon_pm_t h) {
+    double d;
+    std::memcpy(&d, &h->h_words->max_drift, sizeof(double));
+    return d;
 }
 
 // The densest bucket count of the last keying (it picks the deposit form);
 // waits for the work before it.
 int read_max_count(hyowon_pm_t h, uint32_t* out) {
-    CK(cudaMemcpyAsync(h->h_max_count, h->d_max_count, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                       h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    *out = *h->h_max_count;
-    return HYOWON_OK;
+    unsigned int st = 0;
+    const int rc = read_status(h, &st);
+    *out = h->h_words->max_count;
+    return rc;
 }
 
 // Permutes the current particle state into bucket order (used after upload).
@@ -320,11 +331,9 @@ int sort_current(hyowon_pm_t h) {
     CK(cudaMemsetAsync(h->sort.count, 0, sizeof(uint32_t) * (h->sort.n_buckets + 1), h->stream));
     ++h->launches;
     launch_key_f64(n, set_view(h, h->pc, h->mc), h->axis, h->sort, h->d_status, h->stream);
-    h->launches += launch_exclusive_scan(h->sort.count, h->sort.offset, h->sort.n_buckets + 1, h->sort.scan_tmp,
-                          h->stream);
     CK(cudaMemsetAsync(h->d_max_count, 0, sizeof(uint32_t), h->stream));
-    ++h->launches;
-    launch_max_count_f64(h->sort.n_buckets, h->sort.count, h->d_max_count, h->stream);
+    h->launches += launch_exclusive_scan(h->sort.count, h->sort.offset, h->sort.n_buckets + 1,
+                                         h->sort.scan_tmp, h->stream, h->d_max_count);
     const double* src[8];
     double* dst[8];
     int k = 0;
@@ -364,13 +373,11 @@ int index_current(hyowon_pm_t h) {
     CK(cudaMemsetAsync(h->sort.count, 0, sizeof(uint32_t) * (h->sort.n_buckets + 1), h->stream));
     ++h->launches;
     launch_key_f64(n, set_view(h, h->pc, h->mc), h->axis, h->sort, h->d_status, h->stream);
+    CK(cudaMemsetAsync(h->d_max_count, 0, sizeof(uint32_t), h->stream));
     h->launches += launch_exclusive_scan(h->sort.count, h->sort.offset, h->sort.n_buckets + 1,
-                                         h->sort.scan_tmp, h->stream);
+                                         h->sort.scan_tmp, h->stream, h->d_max_count);
     ++h->launches;
     launch_order(n, h->sort.key, h->sort.rank, h->sort.offset, h->order, h->d_status, h->stream);
-    CK(cudaMemsetAsync(h->d_max_count, 0, sizeof(uint32_t), h->stream));
-    ++h->launches;
-    launch_max_count_f64(h->sort.n_buckets, h->sort.count, h->d_max_count, h->stream);
     unsigned int st = 0;
     int rc = read_status(h, &st);
     if (rc) return rc;
@@ -400,14 +407,22 @@ int enqueue_force(hyowon_pm_t h, int pset, int mset, bool kick, double K2,
     }
     const ParticlesF64 p = set_view(h, pset, mset);
     (void)cells;
+    // The densest bucket picks the deposit's form. Up to 128^3 cells both forms are
+    // launched and the device picks: the one that does not apply returns at once
+    // (up to 1024 blocks, 2-3 us), where the host's wait and relaunch leave the
+    // GPU idle for 10 us or more; on larger meshes the empty launch costs as much.
+    const bool device_picks = N <= 128;
     uint32_t max_count = 0;
-    int rc0 = read_max_count(h, &max_count);
-    if (rc0) return rc0;
+    if (!device_picks) {
+        const int rc0 = read_max_count(h, &max_count);
+        if (rc0) return rc0;
+    }
     record(h, 1);
-    ++h->launches;
+    h->launches += device_picks ? 2 : 1;
     // five-pass solve: the deposit writes its tiles transformed along z
     CK(launch_deposit_tiles_f64(p, h->has_masses ? h->mass[h->ic] : nullptr, h->uniform_mass,
-                                order, h->sort, h->axis, h->d_max_count, max_count,
+                                order, h->sort, h->axis, h->d_max_count,
+                                device_picks ? nullptr : &max_count,
                                 deposit_mass_exponent_f64(h->max_mass), h->mesh,
                                 h->five_pass ? h->modes : nullptr, h->tw, h->d_status,
                                 h->stream));
@@ -631,6 +646,7 @@ int kdk_step_impl(hyowon_pm_t h, double K1, double D, double K2, double* max_dri
         int rc = solve_force(h);
         if (rc) return rc;
     }
+    CK(cudaMemsetAsync(h->d_words, 0, sizeof(StepWords), h->stream));
     if (h->precision == HYOWON_FP32_FIXED) {
         int rc = fp32::kdk_step(h->f32, h->stream, h->d_status, h->d_maxdrift, K1, D, K2,
                                 h->timing ? h->ev : nullptr);
@@ -646,20 +662,12 @@ int kdk_step_impl(hyowon_pm_t h, double K1, double D, double K2, double* max_dri
             h->acc_valid = false;
             return status_to_code(h, st);
         }
-        if (max_drift) {
-            CK(cudaMemcpy(h->h_maxdrift, h->d_maxdrift, sizeof(unsigned long long), cudaMemcpyDeviceToHost));
-            double d;
-            std::memcpy(&d, h->h_maxdrift, sizeof(double));
-            *max_drift = d;
-        }
+        if (max_drift) *max_drift = drift_read(h);
         return HYOWON_OK;
     }
     const uint32_t n = h->n;
     const bool sort_now = h->sort_interval <= 1 || h->since_sort + 1 >= h->sort_interval;
-    CK(cudaMemsetAsync(h->d_status, 0, sizeof(unsigned int), h->stream));
-    CK(cudaMemsetAsync(h->d_maxdrift, 0, sizeof(unsigned long long), h->stream));
     CK(cudaMemsetAsync(h->sort.count, 0, sizeof(uint32_t) * (h->sort.n_buckets + 1), h->stream));
-    CK(cudaMemsetAsync(h->d_max_count, 0, sizeof(uint32_t), h->stream));
     record(h, 0);
     // 1. candidate = K1 kick + drift of the current state, into the spare set.
     const ParticlesF64 cur = set_view(h, h->pc, h->mc);
@@ -673,9 +681,7 @@ int kdk_step_impl(hyowon_pm_t h, double K1, double D, double K2, double* max_dri
     int P = 1 - h->pc, M = 1 - h->mc;
     const int ic_before = h->ic;
     h->launches += launch_exclusive_scan(h->sort.count, h->sort.offset, h->sort.n_buckets + 1,
-                                         h->sort.scan_tmp, h->stream);
-    ++h->launches;
-    launch_max_count_f64(h->sort.n_buckets, h->sort.count, h->d_max_count, h->stream);
+                                         h->sort.scan_tmp, h->stream, h->d_max_count);
     const uint32_t* order = nullptr;
     if (!sort_now) {
         ++h->launches;
@@ -732,12 +738,7 @@ int kdk_step_impl(hyowon_pm_t h, double K1, double D, double K2, double* max_dri
     }
     h->mc = 1 - M;  // publish p''
     h->acc_valid = true;
-    if (max_drift) {
-        CK(cudaMemcpy(h->h_maxdrift, h->d_maxdrift, sizeof(unsigned long long), cudaMemcpyDeviceToHost));
-        double d;
-        std::memcpy(&d, h->h_maxdrift, sizeof(double));
-        *max_drift = d;
-    }
+    if (max_drift) *max_drift = drift_read(h);
     return HYOWON_OK;
 }
 
@@ -786,13 +787,14 @@ int hyowon_pm_create(double box_size, uint64_t mesh_size, int method, int deconv
             || cudaEventCreateWithFlags(&h->copied[b], cudaEventDisableTiming) != cudaSuccess)
             return bail(HYOWON_ECUDA);
     }
-    if (cudaMallocHost(reinterpret_cast<void**>(&h->h_status), sizeof(unsigned int)) != cudaSuccess
-        || cudaMallocHost(reinterpret_cast<void**>(&h->h_maxdrift), sizeof(unsigned long long)) != cudaSuccess
-        || cudaMallocHost(reinterpret_cast<void**>(&h->h_max_count), sizeof(uint32_t)) != cudaSuccess
-        || dalloc(&h->d_status, 1) != cudaSuccess || dalloc(&h->d_maxdrift, 1) != cudaSuccess
-        || dalloc(&h->d_max_count, 1) != cudaSuccess
+    if (cudaMallocHost(reinterpret_cast<void**>(&h->h_words), sizeof(StepWords)) != cudaSuccess
+        || dalloc(&h->d_words, 1) != cudaSuccess
+        || cudaMemset(h->d_words, 0, sizeof(StepWords)) != cudaSuccess
         || dalloc(&h->d_diag, diag::scratch_doubles()) != cudaSuccess)
         return bail(HYOWON_ENOMEM);
+    h->d_status = &h->d_words->status;
+    h->d_max_count = &h->d_words->max_count;
+    h->d_maxdrift = &h->d_words->max_drift;
     for (auto& e : h->ev) {
         if (cudaEventCreate(&e) != cudaSuccess) return bail(HYOWON_ECUDA);
     }
@@ -829,7 +831,7 @@ int hyowon_pm_create(double box_size, uint64_t mesh_size, int method, int deconv
 
     if (precision == HYOWON_FP32_FIXED) {
         int rc = fp32::create(&h->f32, h->L, N, method, h->deconvolve, split_scale, lap.data(),
-                              win.data(), h->four_pi_G, h->stream);
+                              win.data(), h->four_pi_G, h->d_max_count, h->stream);
         if (rc) {
             if (h->f32) h->err = fp32::last_error(h->f32);
             return bail(rc);
@@ -905,13 +907,9 @@ int hyowon_pm_destroy(hyowon_pm_t h) {
     cudaFree(h->sort.count);
     cudaFree(h->sort.offset);
     cudaFree(h->sort.scan_tmp);
-    cudaFree(h->d_status);
-    cudaFree(h->d_maxdrift);
-    cudaFree(h->d_max_count);
+    cudaFree(h->d_words);
     cudaFree(h->d_diag);
-    if (h->h_status) cudaFreeHost(h->h_status);
-    if (h->h_max_count) cudaFreeHost(h->h_max_count);
-    if (h->h_maxdrift) cudaFreeHost(h->h_maxdrift);
+    if (h->h_words) cudaFreeHost(h->h_words);
     for (auto& e : h->ev) {
         if (e) cudaEventDestroy(e);
     }
@@ -1401,7 +1399,7 @@ int hyowon_pm_download_mass_mesh(hyowon_pm_t h, double* mesh) {
     ++h->launches;
     CK(launch_deposit_tiles_f64(set_view(h, h->pc, h->mc), h->has_masses ? h->mass[h->ic] : nullptr,
                                 h->uniform_mass, current_order(h), h->sort, h->axis,
-                                h->d_max_count, max_count, deposit_mass_exponent_f64(h->max_mass),
+                                h->d_max_count, &max_count, deposit_mass_exponent_f64(h->max_mass),
                                 h->mesh, nullptr, nullptr, h->d_status, h->stream));
     unsigned int st = 0;
     int rc = read_status(h, &st);

@@ -30,9 +30,10 @@ struct SortWork {
 
 // ---- sort (pm_sort.cu) ----------------------------------------------------
 size_t scan_tmp_elements(uint32_t n_buckets);
-// Returns the number of kernels launched.
+// Returns the number of kernels launched. `most` (may be null): the largest input
+// value is folded into it (atomicMax; the caller zeroes it).
 int launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n,
-                          uint32_t* tmp, cudaStream_t s);
+                          uint32_t* tmp, cudaStream_t s, uint32_t* most = nullptr);
 void launch_scatter_u32(uint32_t n, const uint32_t* key, const uint32_t* rank,
                         const uint32_t* offset, const uint32_t* src, uint32_t* dst,
                         const unsigned int* status, cudaStream_t s);
@@ -72,7 +73,7 @@ void launch_deposit_f64(uint32_t n, const ParticlesF64& p, const double* mass,
 // no zeroing needed. Needs the bucket offsets of the deposited set in w, the
 // cell order `order` (or null when the arrays are in cell order), the largest
 // bucket count in *max_count (and its value on the host, which picks the
-// kernel) and e_max = deposit_mass_exponent_f64(max mass).
+// kernel; null: both forms are launched and the device's value picks) and e_max = deposit_mass_exponent_f64(max mass).
 int deposit_mass_exponent_f64(double max_mass);
 // With `modes` non-null (a power-of-two mesh of 32 to 2048), the tiles are
 // transformed along z and stored to that chunked half spectrum (twiddles `tw`)
@@ -80,11 +81,9 @@ int deposit_mass_exponent_f64(double max_mass);
 cudaError_t launch_deposit_tiles_f64(const ParticlesF64& p, const double* mass,
                                      double uniform_mass, const uint32_t* order,
                                      const SortWork& w, Axis a, const uint32_t* max_count,
-                                     uint32_t max_count_host, int e_max, double* mesh,
+                                     const uint32_t* max_count_host, int e_max, double* mesh,
                                      double2* modes, const double2* tw, unsigned int* status,
                                      cudaStream_t s);
-void launch_max_count_f64(uint32_t n_buckets, const uint32_t* count, uint32_t* max_count,
-                          cudaStream_t s);
 void launch_green_f64(int N, double2* modes, const double* lap, const double* win,
                       double four_pi_G, double scale, int deconvolve, double input_mass,
                       double mass_tolerance, unsigned int* status, cudaStream_t s);

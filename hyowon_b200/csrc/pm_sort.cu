@@ -22,22 +22,11 @@ constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
 constexpr uint32_t kScanTile = kScanThreads * kScanItems;
 
-__global__ void __launch_bounds__(kScanThreads)
-k_scan_block(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32_t n,
-             uint32_t* __restrict__ block_sums) {
-    __shared__ uint32_t warp_tot[kScanThreads / 32];
-    const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    uint32_t sum = 0;
-#pragma unroll
-    for (int j = 0; j < kScanItems; ++j) {
-        v[j] = base + j < n ? in[base + j] : 0u;
-        sum += v[j];
-    }
-    // Inclusive warp scan of the per-thread totals.
+// Block-wide inclusive scan of one value a thread (kScanThreads threads).
+__device__ __forceinline__ uint32_t block_inclusive(uint32_t v, uint32_t* warp_tot) {
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    uint32_t incl = sum;
+    uint32_t incl = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
@@ -55,20 +44,71 @@ k_scan_block(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32
         warp_tot[lane] = w;  // inclusive over warps
     }
     __syncthreads();
-    uint32_t run = incl - sum + (warp > 0 ? warp_tot[warp - 1] : 0u);
-#pragma unroll
-    for (int j = 0; j < kScanItems; ++j) {
-        if (base + j < n) out[base + j] = run;
-        run += v[j];
-    }
-    if (threadIdx.x == kScanThreads - 1 && block_sums) block_sums[blockIdx.x] = run;
+    return incl + (warp > 0 ? warp_tot[warp - 1] : 0u);
 }
 
-__global__ void k_scan_add(uint32_t* __restrict__ out, uint32_t n,
-                           const uint32_t* __restrict__ block_offsets) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    out[i] += block_offsets[i / kScanTile];
+// Exclusive scan of one tile (kScanTile values) per block, or, with `sums` null,
+// of all tiles by one block in turn. The largest value is folded into *most.
+__global__ void __launch_bounds__(kScanThreads)
+k_scan_tiles(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, uint32_t n,
+             uint32_t* __restrict__ sums, uint32_t* __restrict__ most) {
+    __shared__ uint32_t warp_tot[kScanThreads / 32];
+    __shared__ uint32_t total;
+    uint32_t carry = 0, m = 0;
+    for (uint32_t tile = blockIdx.x; static_cast<uint64_t>(tile) * kScanTile < n; ++tile) {
+        const uint32_t base = tile * kScanTile + threadIdx.x * kScanItems;
+        uint32_t v[kScanItems];
+        uint32_t sum = 0;
+#pragma unroll
+        for (int j = 0; j < kScanItems; ++j) {
+            v[j] = base + j < n ? in[base + j] : 0u;
+            sum += v[j];
+            m = max(m, v[j]);
+        }
+        const uint32_t incl = block_inclusive(sum, warp_tot);
+        uint32_t run = carry + incl - sum;
+#pragma unroll
+        for (int j = 0; j < kScanItems; ++j) {
+            if (base + j < n) out[base + j] = run;
+            run += v[j];
+        }
+        if (threadIdx.x == kScanThreads - 1) total = run;
+        __syncthreads();
+        if (sums) {
+            if (threadIdx.x == 0) sums[tile] = total;
+            break;
+        }
+        carry = total;
+        __syncthreads();
+    }
+    if (most) {
+        m = __reduce_max_sync(0xffffffffu, m);
+        if ((threadIdx.x & 31) == 0 && m) atomicMax(most, m);
+    }
+}
+
+// Adds the tiles' offsets: each block sums the totals of the tiles before its own
+// (or, `scanned`, reads their scan).
+__global__ void __launch_bounds__(kScanThreads)
+k_scan_offsets(uint32_t* __restrict__ out, uint32_t n, const uint32_t* __restrict__ sums,
+               int scanned) {
+    __shared__ uint32_t warp_tot[kScanThreads / 32];
+    const uint32_t tile = blockIdx.x + 1;
+    uint32_t add;
+    if (scanned) {
+        add = sums[tile];
+    } else {
+        uint32_t part = 0;
+        for (uint32_t t = threadIdx.x; t < tile; t += kScanThreads) part += sums[t];
+        block_inclusive(part, warp_tot);
+        add = warp_tot[kScanThreads / 32 - 1];
+    }
+    const uint32_t base = tile * kScanTile + threadIdx.x;
+#pragma unroll
+    for (int j = 0; j < kScanItems; ++j) {
+        const uint32_t i = base + j * kScanThreads;
+        if (i < n) out[i] += add;
+    }
 }
 
 // Permute up to 8 binary64 arrays and 2 u32 arrays in one pass.
@@ -158,31 +198,26 @@ size_t scan_tmp_elements(uint32_t n) {
 }
 
 int launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* tmp,
-                          cudaStream_t s) {
-    if (n == 0) return 0;
-    const uint32_t nb = static_cast<uint32_t>((static_cast<uint64_t>(n) + kScanTile - 1) / kScanTile);
-    if (nb == 1) {
-        k_scan_block<<<1, kScanThreads, 0, s>>>(in, out, n, nullptr);
+                          cudaStream_t s, uint32_t* most) {
+    const uint32_t tiles = blocks_for(n, kScanTile);
+    // One block up to four tiles: three launches of some 3 us each for the
+    // 4097 bucket counts of a 64^3 mesh became one.
+    if (tiles <= 4) {
+        k_scan_tiles<<<1, kScanThreads, 0, s>>>(in, out, n, nullptr, most);
         return 1;
     }
     uint32_t* sums = tmp;
-    uint32_t* sums_scanned = tmp + nb + 32;
-    k_scan_block<<<nb, kScanThreads, 0, s>>>(in, out, n, sums);
-    const int inner = launch_exclusive_scan(sums, sums_scanned, nb, tmp + 2 * nb + 64, s);
-    k_scan_add<<<blocks_for(n, 256), 256, 0, s>>>(out, n, sums_scanned);
-    return inner + 2;
-}
-
-void launch_scatter_f64(uint32_t n, const uint32_t* key, const uint32_t* rank,
-                        const uint32_t* offset, const double* src, double* dst,
-                        const unsigned int* status, cudaStream_t s) {
-    if (n == 0) return;
-    ScatterArrays a{};
-    a.src[0] = src;
-    a.dst[0] = dst;
-    a.n_f64 = 1;
-    a.n_u32 = 0;
-    k_scatter<<<blocks_for(n, 256), 256, 0, s>>>(n, key, rank, offset, a, status);
+    k_scan_tiles<<<tiles, kScanThreads, 0, s>>>(in, out, n, sums, most);
+    // Every block sums the totals before its tile itself while that is a few
+    // thousand values from L2; beyond that they are scanned first.
+    if (tiles <= 8192) {
+        k_scan_offsets<<<tiles - 1, kScanThreads, 0, s>>>(out, n, sums, 0);
+        return 2;
+    }
+    uint32_t* sums_scanned = tmp + tiles + 32;
+    const int inner = launch_exclusive_scan(sums, sums_scanned, tiles, tmp + 2 * tiles + 64, s, nullptr);
+    k_scan_offsets<<<tiles - 1, kScanThreads, 0, s>>>(out, n, sums_scanned, 1);
+    return 2 + inner;
 }
 
 void launch_scatter_u32(uint32_t n, const uint32_t* key, const uint32_t* rank,
