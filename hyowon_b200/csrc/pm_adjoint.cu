@@ -91,6 +91,18 @@ __device__ __forceinline__ size_t cidx(int x, int y, int z, int N) {
 __device__ __forceinline__ int up(int i, int N) { return i + 1 == N ? 0 : i + 1; }
 __device__ __forceinline__ int dn(int i, int N) { return i == 0 ? N - 1 : i - 1; }
 
+// Adds m * w to the 8 corner cells of a particle.
+template <typename R>
+__device__ __forceinline__ void deposit_corners(const Corner& c, R m, int N, R* __restrict__ mesh) {
+    const R wx[2] = {R(1) - R(c.fx), R(c.fx)}, wy[2] = {R(1) - R(c.fy), R(c.fy)},
+            wz[2] = {R(1) - R(c.fz), R(c.fz)};
+    const int gx[2] = {c.ix, up(c.ix, N)}, gy[2] = {c.iy, up(c.iy, N)}, gz[2] = {c.iz, up(c.iz, N)};
+    for (int u = 0; u < 2; ++u)
+        for (int v = 0; v < 2; ++v)
+            for (int w = 0; w < 2; ++w)
+                atomicAdd(&mesh[cidx(gx[u], gy[v], gz[w], N)], m * wx[u] * wy[v] * wz[w]);
+}
+
 template <typename R>
 __global__ void k_deposit(uint32_t n, const double* __restrict__ x, const double* __restrict__ y,
                           const double* __restrict__ z, R m, Axis a, R* __restrict__ mesh,
@@ -102,17 +114,11 @@ __global__ void k_deposit(uint32_t n, const double* __restrict__ x, const double
         raise_status(status, ST_CELL_ESCAPE);
         return;
     }
-    const int N = a.N;
-    const R wx[2] = {R(1) - R(c.fx), R(c.fx)}, wy[2] = {R(1) - R(c.fy), R(c.fy)},
-            wz[2] = {R(1) - R(c.fz), R(c.fz)};
-    const int gx[2] = {c.ix, up(c.ix, N)}, gy[2] = {c.iy, up(c.iy, N)}, gz[2] = {c.iz, up(c.iz, N)};
-    for (int u = 0; u < 2; ++u)
-        for (int v = 0; v < 2; ++v)
-            for (int w = 0; w < 2; ++w)
-                atomicAdd(&mesh[cidx(gx[u], gy[v], gz[w], N)], m * wx[u] * wy[v] * wz[w]);
+    deposit_corners(c, m, a.N, mesh);
 }
 
-// Three-component CIC scatter (transpose of the interpolation). Particles
+// Three-component CIC scatter (transpose of the interpolation) of the force
+// cotangent coef * l. Particles
 // stay in lattice order, so consecutive lanes usually hold z-neighbours in the
 // same (x, y) cell column: when lane l+1's lower z cells are lane l's upper z
 // cells, lane l hands its upper-z weights to lane l+1, which adds them to its
@@ -120,9 +126,10 @@ __global__ void k_deposit(uint32_t n, const double* __restrict__ x, const double
 // the same up to the order of additions, which atomics leave open anyway).
 template <typename R>
 __global__ void k_scatter3(uint32_t n, const double* __restrict__ x, const double* __restrict__ y,
-                           const double* __restrict__ z, const R* __restrict__ v0,
-                           const R* __restrict__ v1, const R* __restrict__ v2, Axis a,
-                           R* __restrict__ u0, R* __restrict__ u1, R* __restrict__ u2) {
+                           const double* __restrict__ z, const double* __restrict__ l0,
+                           const double* __restrict__ l1, const double* __restrict__ l2,
+                           double coef, Axis a, R* __restrict__ u0, R* __restrict__ u1,
+                           R* __restrict__ u2) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const int N = a.N;
@@ -137,7 +144,8 @@ __global__ void k_scatter3(uint32_t n, const double* __restrict__ x, const doubl
         gx[0] = c.ix; gx[1] = up(c.ix, N);
         gy[0] = c.iy; gy[1] = up(c.iy, N);
         gz[0] = c.iz; gz[1] = up(c.iz, N);
-        const R av[3] = {v0[i], v1[i], v2[i]};
+        const R av[3] = {static_cast<R>(coef * l0[i]), static_cast<R>(coef * l1[i]),
+                         static_cast<R>(coef * l2[i])};
         for (int u = 0; u < 2; ++u)
             for (int v = 0; v < 2; ++v)
                 for (int d = 0; d < 3; ++d) {
@@ -257,32 +265,70 @@ __device__ __forceinline__ bool force_at(double px, double py, double pz, const 
     return true;
 }
 
-// One step of the reverse leapfrog between re-solves: x = wrap(x - D p_half),
-// a = F(x) from the potential the forward pass kept for that state,
-// p = p_half - K1 a (the inverse of kick K1 + drift D).
+// One forward step of a particle at x_j, whose potential is known: a = F(x_j), the
+// closing kick K2 of the step before (K2 = 0 at the start), the state to the
+// checkpoint arrays when given, then, when `more`, the opening kick K1, the drift
+// and the deposit at x_{j+1} into the zeroed `mesh`; else a to the acceleration
+// arrays. One pass over the particles in place of force, two kicks, drift, deposit
+// and the checkpoint's copies, each of which re-read what the last wrote: the
+// forward pass of 16 steps at 128^3 takes 3.67 ms (4.56), of 8 steps at 48^3 on a
+// 96^3 mesh in FP32 0.62 (0.81). The loads of the stencil bound it.
 template <typename R>
-__global__ void k_unstep(uint32_t n, double* __restrict__ x0, double* __restrict__ x1,
-                         double* __restrict__ x2, R* __restrict__ p0, R* __restrict__ p1,
-                         R* __restrict__ p2, double D, double L, const R* __restrict__ phi, Axis a,
-                         R inv_two_dx, R K1, R* __restrict__ ax, R* __restrict__ ay,
-                         R* __restrict__ az) {
+struct Checkpoint {
+    double* x[3];
+    R* p[3];
+};
+template <typename R>
+__global__ void __launch_bounds__(kT)
+k_advance(uint32_t n, double* __restrict__ x0, double* __restrict__ x1, double* __restrict__ x2,
+          R* __restrict__ p0, R* __restrict__ p1, R* __restrict__ p2, const R* __restrict__ phi,
+          Axis a, R inv_two_dx, R K2, Checkpoint<R> save, int more, R K1, double D, R m,
+          R* __restrict__ mesh, R* __restrict__ ax, R* __restrict__ ay, R* __restrict__ az,
+          unsigned int* status) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const R q0 = p0[i], q1 = p1[i], q2 = p2[i];
-    const double nx = wrap_f64(x0[i] + D * static_cast<double>(q0), L);
-    const double ny = wrap_f64(x1[i] + D * static_cast<double>(q1), L);
-    const double nz = wrap_f64(x2[i] + D * static_cast<double>(q2), L);
+    const double x = x0[i], y = x1[i], z = x2[i];
+    R q0 = p0[i], q1 = p1[i], q2 = p2[i];
+    R s0, s1, s2;
+    if (!force_at(x, y, z, phi, a, inv_two_dx, s0, s1, s2)) return;   // raised by the deposit
+    q0 += K2 * s0;
+    q1 += K2 * s1;
+    q2 += K2 * s2;
+    if (save.x[0]) {
+        save.x[0][i] = x;
+        save.x[1][i] = y;
+        save.x[2][i] = z;
+        save.p[0][i] = q0;
+        save.p[1][i] = q1;
+        save.p[2][i] = q2;
+    }
+    if (!more) {
+        ax[i] = s0;
+        ay[i] = s1;
+        az[i] = s2;
+        p0[i] = q0;
+        p1[i] = q1;
+        p2[i] = q2;
+        return;
+    }
+    q0 += K1 * s0;
+    q1 += K1 * s1;
+    q2 += K1 * s2;
+    const double nx = wrap_f64(x + D * static_cast<double>(q0), a.L);
+    const double ny = wrap_f64(y + D * static_cast<double>(q1), a.L);
+    const double nz = wrap_f64(z + D * static_cast<double>(q2), a.L);
     x0[i] = nx;
     x1[i] = ny;
     x2[i] = nz;
-    R s0, s1, s2;
-    if (!force_at(nx, ny, nz, phi, a, inv_two_dx, s0, s1, s2)) return;
-    ax[i] = s0;
-    ay[i] = s1;
-    az[i] = s2;
-    p0[i] = q0 + K1 * s0;
-    p1[i] = q1 + K1 * s1;
-    p2[i] = q2 + K1 * s2;
+    p0[i] = q0;
+    p1[i] = q1;
+    p2[i] = q2;
+    Corner c;
+    if (!corner_of(nx, ny, nz, a, c)) {
+        raise_status(status, ST_CELL_ESCAPE);
+        return;
+    }
+    deposit_corners(c, m, a.N, mesh);
 }
 
 // lp += D lx (the drift's transpose) and p += K a (a kick), one pass.
@@ -329,41 +375,130 @@ __global__ void k_force(uint32_t n, const double* __restrict__ x, const double* 
     az[i] = s2;
 }
 
-// out_j += sum_c dW_jc/dx_j (mpsi * psi_c + v_j . g_c)   (phi / v may be null)
+// d(v.F)/dx of one particle: sum_c dW_c/dx (mpsi psi_c + v . g_c); phi may be null
+// (v = 0).
+template <typename R>
+__device__ __forceinline__ void force_vjp(const Corner& c, int N, const R* __restrict__ psi, R mpsi,
+                                          const R* __restrict__ phi, const R (&vv)[3],
+                                          R inv_two_dx, R& s0, R& s1, R& s2) {
+    R g[2][2][2][3];
+    const bool with_v = phi != nullptr;
+    if (with_v) corner_forces(phi, c, N, inv_two_dx, g);
+    const R inv_dx = R(2) * inv_two_dx;
+    const R wx[2] = {R(1) - R(c.fx), R(c.fx)}, wy[2] = {R(1) - R(c.fy), R(c.fy)},
+            wz[2] = {R(1) - R(c.fz), R(c.fz)};
+    const R dw[2] = {-inv_dx, inv_dx};
+    const int gx[2] = {c.ix, up(c.ix, N)}, gy[2] = {c.iy, up(c.iy, N)}, gz[2] = {c.iz, up(c.iz, N)};
+    s0 = s1 = s2 = 0;
+    for (int u = 0; u < 2; ++u)
+        for (int v = 0; v < 2; ++v)
+            for (int w = 0; w < 2; ++w) {
+                R h = mpsi * psi[cidx(gx[u], gy[v], gz[w], N)];
+                if (with_v) h += vv[0] * g[u][v][w][0] + vv[1] * g[u][v][w][1] + vv[2] * g[u][v][w][2];
+                s0 += dw[u] * wy[v] * wz[w] * h;
+                s1 += wx[u] * dw[v] * wz[w] * h;
+                s2 += wx[u] * wy[v] * dw[w] * h;
+            }
+}
+
+// lx += d(v.F)/dx with v = coef * lp (phi null: the density loss alone).
 template <typename R>
 __global__ void k_vjp_gather(uint32_t n, const double* __restrict__ x, const double* __restrict__ y,
                              const double* __restrict__ z, const R* __restrict__ psi, R mpsi,
-                             const R* __restrict__ phi, const R* __restrict__ v0,
-                             const R* __restrict__ v1, const R* __restrict__ v2, Axis a,
+                             const R* __restrict__ phi, double coef, const double* __restrict__ l0,
+                             const double* __restrict__ l1, const double* __restrict__ l2, Axis a,
                              R inv_two_dx, double* __restrict__ o0, double* __restrict__ o1,
                              double* __restrict__ o2) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     Corner c;
     if (!corner_of(x[i], y[i], z[i], a, c)) return;
-    const int N = a.N;
-    R g[2][2][2][3];
-    const bool with_v = phi != nullptr;
-    if (with_v) corner_forces(phi, c, N, inv_two_dx, g);
-    const R vv[3] = {with_v ? v0[i] : R(0), with_v ? v1[i] : R(0), with_v ? v2[i] : R(0)};
-    const R inv_dx = R(2) * inv_two_dx;
-    const R wx[2] = {R(1) - R(c.fx), R(c.fx)}, wy[2] = {R(1) - R(c.fy), R(c.fy)},
-            wz[2] = {R(1) - R(c.fz), R(c.fz)};
-    const R dw[2] = {-inv_dx, inv_dx};
-    const int gx[2] = {c.ix, up(c.ix, N)}, gy[2] = {c.iy, up(c.iy, N)}, gz[2] = {c.iz, up(c.iz, N)};
-    R s0 = 0, s1 = 0, s2 = 0;
-    for (int u = 0; u < 2; ++u)
-        for (int v = 0; v < 2; ++v)
-            for (int w = 0; w < 2; ++w) {
-                R h = psi ? mpsi * psi[cidx(gx[u], gy[v], gz[w], N)] : R(0);
-                if (with_v) h += vv[0] * g[u][v][w][0] + vv[1] * g[u][v][w][1] + vv[2] * g[u][v][w][2];
-                s0 += dw[u] * wy[v] * wz[w] * h;
-                s1 += wx[u] * dw[v] * wz[w] * h;
-                s2 += wx[u] * wy[v] * dw[w] * h;
-            }
+    R vv[3] = {R(0), R(0), R(0)};
+    if (phi) {
+        vv[0] = static_cast<R>(coef * l0[i]);
+        vv[1] = static_cast<R>(coef * l1[i]);
+        vv[2] = static_cast<R>(coef * l2[i]);
+    }
+    R s0, s1, s2;
+    force_vjp(c, a.N, psi, mpsi, phi, vv, inv_two_dx, s0, s1, s2);
     o0[i] += static_cast<double>(s0);
     o1[i] += static_cast<double>(s1);
     o2[i] += static_cast<double>(s2);
+}
+
+// One reverse step of a particle from x_{j+1} to x_j where the forward pass kept
+// both potentials: lx += d(v.F)/dx at x_{j+1} (v = coef lp), lp += D lx, the kick
+// K2 undone, then either the checkpointed state or the drift D undone, a = F(x_j)
+// from its potential, and the kick K1 undone. One pass in place of the gather, the
+// axpy / kick and the un-step or the checkpoint's copies and force; with the
+// scatter's and the gather's cotangents formed in place the reverse pass of the same
+// runs takes 7.33 ms (8.56) and 0.91 (1.06).
+template <typename R>
+__global__ void __launch_bounds__(kT)
+k_reverse(uint32_t n, double* __restrict__ x0, double* __restrict__ x1, double* __restrict__ x2,
+          R* __restrict__ p0, R* __restrict__ p1, R* __restrict__ p2, R* __restrict__ ax,
+          R* __restrict__ ay, R* __restrict__ az, const R* __restrict__ psi, R mpsi,
+          const R* __restrict__ phi_next, const R* __restrict__ phi, double coef, double D, R K1,
+          R K2, Checkpoint<R> from, Axis a, R inv_two_dx, double* __restrict__ lx0,
+          double* __restrict__ lx1, double* __restrict__ lx2, double* __restrict__ lp0,
+          double* __restrict__ lp1, double* __restrict__ lp2) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const double x = x0[i], y = x1[i], z = x2[i];
+    const double k0 = lp0[i], k1 = lp1[i], k2 = lp2[i];
+    double g0 = lx0[i], g1 = lx1[i], g2 = lx2[i];
+    {
+        Corner c;
+        if (corner_of(x, y, z, a, c)) {
+            const R vv[3] = {static_cast<R>(coef * k0), static_cast<R>(coef * k1),
+                             static_cast<R>(coef * k2)};
+            R s0, s1, s2;
+            force_vjp(c, a.N, psi, mpsi, phi_next, vv, inv_two_dx, s0, s1, s2);
+            g0 += static_cast<double>(s0);
+            g1 += static_cast<double>(s1);
+            g2 += static_cast<double>(s2);
+            lx0[i] = g0;
+            lx1[i] = g1;
+            lx2[i] = g2;
+        }
+    }
+    lp0[i] = k0 + D * g0;
+    lp1[i] = k1 + D * g1;
+    lp2[i] = k2 + D * g2;
+    double nx, ny, nz;
+    R q0, q1, q2;
+    if (from.x[0]) {
+        nx = from.x[0][i];
+        ny = from.x[1][i];
+        nz = from.x[2][i];
+        q0 = from.p[0][i];
+        q1 = from.p[1][i];
+        q2 = from.p[2][i];
+    } else {
+        q0 = p0[i] - K2 * ax[i];
+        q1 = p1[i] - K2 * ay[i];
+        q2 = p2[i] - K2 * az[i];
+        nx = wrap_f64(x - D * static_cast<double>(q0), a.L);
+        ny = wrap_f64(y - D * static_cast<double>(q1), a.L);
+        nz = wrap_f64(z - D * static_cast<double>(q2), a.L);
+    }
+    x0[i] = nx;
+    x1[i] = ny;
+    x2[i] = nz;
+    R s0, s1, s2;
+    if (force_at(nx, ny, nz, phi, a, inv_two_dx, s0, s1, s2)) {
+        ax[i] = s0;
+        ay[i] = s1;
+        az[i] = s2;
+        if (!from.x[0]) {
+            q0 -= K1 * s0;
+            q1 -= K1 * s1;
+            q2 -= K1 * s2;
+        }
+    }
+    p0[i] = q0;
+    p1[i] = q1;
+    p2[i] = q2;
 }
 
 template <typename R>
@@ -386,18 +521,6 @@ __global__ void k_drift(uint32_t n, double* __restrict__ x0, double* __restrict_
     x0[i] = wrap_f64(x0[i] + D * static_cast<double>(p0[i]), L);
     x1[i] = wrap_f64(x1[i] + D * static_cast<double>(p1[i]), L);
     x2[i] = wrap_f64(x2[i] + D * static_cast<double>(p2[i]), L);
-}
-
-// v = coef * lp (as Real) ; lp += D * lx
-template <typename R>
-__global__ void k_cotangent(uint32_t n, const double* __restrict__ l0, const double* __restrict__ l1,
-                            const double* __restrict__ l2, double coef, R* __restrict__ v0,
-                            R* __restrict__ v1, R* __restrict__ v2) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    v0[i] = static_cast<R>(coef * l0[i]);
-    v1[i] = static_cast<R>(coef * l1[i]);
-    v2[i] = static_cast<R>(coef * l2[i]);
 }
 
 __global__ void k_axpy3(uint32_t n, double a, const double* __restrict__ x0,
@@ -616,10 +739,9 @@ public:
         for (void* p : owned_) cudaFree(p);
     }
 
-    // acc = F(x); phi_ = potential at x, written to `keep` when given (the
-    // forward pass's copy of it), else to the engine's own mesh.
-    void force(R* keep = nullptr) {
-        phi_ = keep ? keep : phi_own_;
+    // acc = F(x); phi_ = potential at x, in the engine's own mesh.
+    void force() {
+        phi_ = phi_own_;
         ACK(cudaMemsetAsync(mesh_, 0, sizeof(R) * cells_, s_));
         k_deposit<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], static_cast<R>(cfg_.particle_mass),
                                             axis_, mesh_, status_);
@@ -627,13 +749,6 @@ public:
         k_force<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], phi_, axis_, inv_two_dx_, acc_[0],
                                           acc_[1], acc_[2]);
         ++solves_;
-    }
-
-    // acc = F(x) from a potential the forward pass kept for this state.
-    void force_from(R* kept) {
-        phi_ = kept;
-        k_force<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], phi_, axis_, inv_two_dx_, acc_[0],
-                                          acc_[1], acc_[2]);
     }
 
     // out = A in: r2c, Green's function (k = 0 zeroed), c2r with 1/N^3. On
@@ -673,18 +788,22 @@ public:
         k_drift<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], p_[0], p_[1], p_[2], D, cfg_.box_size);
     }
 
-    // lx += VJP_F(x; v), v = coef * lp
-    void vjp(double coef, double* const lx[3], double* const lp[3], R* const v[3], R* const u[3], R* psi) {
-        k_cotangent<R><<<nb(n_), kT, 0, s_>>>(n_, lp[0], lp[1], lp[2], coef, v[0], v[1], v[2]);
+    // psi = A div(scatter(coef * lp)): the mesh half of VJP_F at x.
+    void vjp_mesh(double coef, double* const lp[3], R* const u[3], R* psi) {
         for (int a = 0; a < 3; ++a) ACK(cudaMemsetAsync(u[a], 0, sizeof(R) * cells_, s_));
-        k_scatter3<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], v[0], v[1], v[2], axis_, u[0],
-                                             u[1], u[2]);
+        k_scatter3<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], lp[0], lp[1], lp[2], coef, axis_,
+                                             u[0], u[1], u[2]);
         k_divergence<R><<<nb(cells_), kT, 0, s_>>>(N_, u[0], u[1], u[2], inv_two_dx_, mesh_);
         apply_green(mesh_, psi);
-        k_vjp_gather<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], psi,
-                                               static_cast<R>(cfg_.particle_mass), phi_, v[0], v[1],
-                                               v[2], axis_, inv_two_dx_, lx[0], lx[1], lx[2]);
         ++vjps_;
+    }
+
+    // lx += VJP_F(x; coef * lp)
+    void vjp(double coef, double* const lx[3], double* const lp[3], R* const u[3], R* psi) {
+        vjp_mesh(coef, lp, u, psi);
+        k_vjp_gather<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], psi,
+                                               static_cast<R>(cfg_.particle_mass), phi_, coef, lp[0],
+                                               lp[1], lp[2], axis_, inv_two_dx_, lx[0], lx[1], lx[2]);
     }
 
     void run(const double* noise, const double* target, double* loss_out, double* grad_out,
@@ -701,7 +820,7 @@ public:
         double *d_noise = nullptr, *tab = nullptr, *d_loss = nullptr, *d_delta = nullptr,
                *d_target = nullptr, *grad = nullptr;
         double *pd[3], *lx[3] = {}, *lp[3] = {};
-        R *v[3] = {}, *u[3] = {}, *psi = nullptr, *field = nullptr, *kept_block = nullptr;
+        R *u[3] = {}, *psi = nullptr, *field = nullptr, *kept_block = nullptr;
         std::vector<double*> cx(3 * n_ckpt);
         std::vector<R*> cp(3 * n_ckpt);
         bool keep = false;
@@ -717,7 +836,6 @@ public:
                 for (int a = 0; a < 3; ++a) {
                     lx[a] = arena_.template take<double>(n_);
                     lp[a] = arena_.template take<double>(n_);
-                    v[a] = arena_.template take<R>(n_);
                     u[a] = arena_.template take<R>(cells_);
                 }
                 psi = arena_.template take<R>(cells_);
@@ -763,11 +881,13 @@ public:
         if (keep)
             for (uint64_t j = 0; j <= S; ++j) kept.push_back(kept_block + j * phi_stride);
         auto keep_of = [&](uint64_t j) { return kept.empty() ? nullptr : kept[j]; };
-        auto save = [&](uint64_t c) {
+        auto checkpoint = [&](uint64_t c) {
+            Checkpoint<R> k;
             for (int a = 0; a < 3; ++a) {
-                ACK(cudaMemcpyAsync(cx[3 * c + a], x_[a], sizeof(double) * n_, cudaMemcpyDeviceToDevice, s_));
-                ACK(cudaMemcpyAsync(cp[3 * c + a], p_[a], sizeof(R) * n_, cudaMemcpyDeviceToDevice, s_));
+                k.x[a] = cx[3 * c + a];
+                k.p[a] = cp[3 * c + a];
             }
+            return k;
         };
         auto restore = [&](uint64_t c) {
             for (int a = 0; a < 3; ++a) {
@@ -793,21 +913,26 @@ public:
         // Timed: the KDK forward from the 1LPT state, the loss, and the reverse
         // KDK pass (the 1LPT map and its adjoint, one FFT set each, are setup).
         cudaEventRecord(e0, s_);
-        force(keep_of(0));
-        save(0);
-        for (uint64_t j = 0; j < S; ++j) {
-            kick(cfg_.K1[j]);
-            drift(cfg_.D[j]);
-            force(keep_of(j + 1));
-            kick(cfg_.K2[j]);
-            if ((j + 1) % k == 0 && j + 1 < S) save((j + 1) / k);
+        ACK(cudaMemsetAsync(mesh_, 0, sizeof(R) * cells_, s_));
+        k_deposit<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], static_cast<R>(cfg_.particle_mass),
+                                            axis_, mesh_, status_);
+        for (uint64_t j = 0; j <= S; ++j) {
+            // potential of state j from its deposit, then the step to state j + 1
+            phi_ = keep_of(j) ? keep_of(j) : phi_own_;
+            apply_green(mesh_, phi_);
+            ++solves_;
+            if (j < S) ACK(cudaMemsetAsync(mesh_, 0, sizeof(R) * cells_, s_));
+            k_advance<R><<<nb(n_), kT, 0, s_>>>(
+                n_, x_[0], x_[1], x_[2], p_[0], p_[1], p_[2], phi_, axis_, inv_two_dx_,
+                static_cast<R>(j > 0 ? cfg_.K2[j - 1] : 0.0),
+                j % k == 0 && j < S ? checkpoint(j / k) : Checkpoint<R>{}, j < S ? 1 : 0,
+                static_cast<R>(j < S ? cfg_.K1[j] : 0.0), j < S ? cfg_.D[j] : 0.0,
+                static_cast<R>(cfg_.particle_mass), mesh_, acc_[0], acc_[1], acc_[2], status_);
         }
         // ---- loss on the final CIC density ----------------------------------
         const double mbar = cfg_.particle_mass * static_cast<double>(n_) / static_cast<double>(cells_);
         ACK(cudaMemsetAsync(d_loss, 0, sizeof(double), s_));
-        ACK(cudaMemsetAsync(mesh_, 0, sizeof(R) * cells_, s_));
-        k_deposit<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], static_cast<R>(cfg_.particle_mass),
-                                            axis_, mesh_, status_);
+        // mesh_ still holds the deposit of the last state: the solve reads it only
         k_loss<R><<<1184, kT, 0, s_>>>(cells_, mesh_, d_target, 1.0 / mbar, cfg_.particle_mass / mbar,
                                        field, d_delta, d_loss);
         ACK(cudaMemcpyAsync(loss_out, d_loss, sizeof(double), cudaMemcpyDeviceToHost, s_));
@@ -821,32 +946,37 @@ public:
                 ACK(cudaMemsetAsync(lp[a], 0, sizeof(double) * n_, s_));
             }
             // dL/dx_S: deposit transpose with the weight derivative.
-            k_vjp_gather<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], field, R(1), nullptr,
+            k_vjp_gather<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], field, R(1), nullptr, 0.0,
                                                    nullptr, nullptr, nullptr, axis_, inv_two_dx_,
                                                    lx[0], lx[1], lx[2]);
             for (uint64_t jj = S; jj-- > 0;) {
                 const double coef = cfg_.K2[jj] + (jj + 1 < S ? cfg_.K1[jj + 1] : 0.0);
-                vjp(coef, lx, lp, v, u, psi);  // at x_{jj+1} with phi_{jj+1}
+                if (!kept.empty()) {
+                    vjp_mesh(coef, lp, u, psi);   // at x_{jj+1}
+                    k_reverse<R><<<nb(n_), kT, 0, s_>>>(
+                        n_, x_[0], x_[1], x_[2], p_[0], p_[1], p_[2], acc_[0], acc_[1], acc_[2], psi,
+                        static_cast<R>(cfg_.particle_mass), kept[jj + 1], kept[jj], coef, cfg_.D[jj],
+                        static_cast<R>(cfg_.K1[jj]), static_cast<R>(cfg_.K2[jj]),
+                        jj % k == 0 ? checkpoint(jj / k) : Checkpoint<R>{}, axis_, inv_two_dx_, lx[0],
+                        lx[1], lx[2], lp[0], lp[1], lp[2]);
+                    phi_ = kept[jj];
+                    continue;
+                }
+                vjp(coef, lx, lp, u, psi);  // at x_{jj+1} with phi_{jj+1}
                 // lp += D lx; reconstruct state jj: p' = p_{jj+1} - K2 a_{jj+1}
                 k_axpy3_kick<R><<<nb(n_), kT, 0, s_>>>(n_, cfg_.D[jj], lx[0], lx[1], lx[2], lp[0],
                                                        lp[1], lp[2], p_[0], p_[1], p_[2], acc_[0],
                                                        acc_[1], acc_[2], static_cast<R>(-cfg_.K2[jj]));
                 if (jj % k == 0) {
                     restore(jj / k);
-                    if (kept.empty()) force(); else force_from(kept[jj]);
-                } else if (kept.empty()) {
+                    force();
+                } else {
                     drift(-cfg_.D[jj]);
                     force();
                     kick(-cfg_.K1[jj]);
-                } else {
-                    phi_ = kept[jj];
-                    k_unstep<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], p_[0], p_[1], p_[2],
-                                                       -cfg_.D[jj], cfg_.box_size, phi_, axis_,
-                                                       inv_two_dx_, static_cast<R>(-cfg_.K1[jj]),
-                                                       acc_[0], acc_[1], acc_[2]);
                 }
             }
-            vjp(cfg_.K1[0], lx, lp, v, u, psi);  // at x_0
+            vjp(cfg_.K1[0], lx, lp, u, psi);  // at x_0
             cudaEventRecord(e2, s_);
             // ---- 1LPT adjoint: g_d = lx_d + pf lp_d -----------------------------
             k_axpy3<<<nb(n_), kT, 0, s_>>>(n_, cfg_.momentum_factor, lp[0], lp[1], lp[2], lx[0],
