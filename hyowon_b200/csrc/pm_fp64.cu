@@ -44,13 +44,19 @@ inline bool cells_fit_u32(int N) {
     return static_cast<uint64_t>(N) * N * N <= 0xffffffffull;
 }
 
-__global__ void k_validate_inputs(uint32_t n, const double* __restrict__ x,
-                                  const double* __restrict__ y,
-                                  const double* __restrict__ z,
-                                  const double* __restrict__ mass,
-                                  unsigned int* status) {
+// What an upload does besides the copies, in one pass: the input checks, the
+// particles' ids, and zero momenta where none were given (px null: given).
+__global__ void k_accept_upload(uint32_t n, const double* __restrict__ x,
+                                const double* __restrict__ y, const double* __restrict__ z,
+                                const double* __restrict__ mass, uint32_t* __restrict__ id,
+                                double* __restrict__ px, double* __restrict__ py,
+                                double* __restrict__ pz, unsigned int* status) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    id[i] = i;
+    if (px) px[i] = 0.0;
+    if (py) py[i] = 0.0;
+    if (pz) pz[i] = 0.0;
     bool bad = !isfinite(x[i]) || !isfinite(y[i]) || !isfinite(z[i]);
     if (mass) bad |= !isfinite(mass[i]) || mass[i] < 0.0;
     if (bad) raise_status(status, ST_NONFINITE_INPUT);
@@ -814,11 +820,11 @@ __global__ void k_cell_coords(uint32_t n, const double* __restrict__ pos, Axis a
 
 }  // namespace
 
-void launch_validate_inputs_f64(uint32_t n, const double* x, const double* y,
-                                const double* z, const double* mass, unsigned int* status,
-                                cudaStream_t s) {
+void launch_accept_upload_f64(uint32_t n, const double* x, const double* y, const double* z,
+                              const double* mass, uint32_t* id, double* px, double* py, double* pz,
+                              unsigned int* status, cudaStream_t s) {
     if (n == 0) return;
-    k_validate_inputs<<<blocks_for(n), kThreads, 0, s>>>(n, x, y, z, mass, status);
+    k_accept_upload<<<blocks_for(n), kThreads, 0, s>>>(n, x, y, z, mass, id, px, py, pz, status);
 }
 
 void launch_key_f64(uint32_t n, const ParticlesF64& p, Axis a, const SortWork& w,

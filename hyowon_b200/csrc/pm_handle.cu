@@ -325,8 +325,18 @@ int read_max_count(hyowon_pm_t h, uint32_t* out) {
     return rc;
 }
 
-// Permutes the current particle state into bucket order (used after upload).
-int sort_current(hyowon_pm_t h) {
+// Exchanges the particle buffer sets (after a sort, or to undo one).
+void swap_sets(hyowon_pm_t h) {
+    h->pc = 1 - h->pc;
+    h->mc = 1 - h->mc;
+    h->ic = 1 - h->ic;
+}
+
+// Permutes the current particle state into bucket order (used after upload). With
+// `defer` the status is left for the caller to read after the solve that follows:
+// a failed keying blocks the scatter and every later write, and the caller swaps
+// the sets back.
+int sort_current(hyowon_pm_t h, bool defer = false) {
     const uint32_t n = h->n;
     CK(cudaMemsetAsync(h->sort.count, 0, sizeof(uint32_t) * (h->sort.n_buckets + 1), h->stream));
     ++h->launches;
@@ -354,13 +364,13 @@ int sort_current(hyowon_pm_t h) {
     ++h->launches;
     launch_scatter_multi(n, h->sort.key, h->sort.rank, h->sort.offset, k, src, dst, 1, su, du,
                          h->d_status, h->stream);
-    unsigned int st = 0;
-    int rc = read_status(h, &st);
-    if (rc) return rc;
-    if (st) return status_to_code(h, st);
-    h->pc = 1 - h->pc;
-    h->mc = 1 - h->mc;
-    h->ic = 1 - h->ic;
+    if (!defer) {
+        unsigned int st = 0;
+        int rc = read_status(h, &st);
+        if (rc) return rc;
+        if (st) return status_to_code(h, st);
+    }
+    swap_sets(h);
     h->sorted = true;
     h->order_state = 1;
     return HYOWON_OK;
@@ -599,17 +609,22 @@ int short_range_hook_f32(void* ctx, cudaStream_t s, int P) {
 
 // Force solve at the current positions; accelerations become valid.
 int solve_force(hyowon_pm_t h) {
-    if (!h->sorted) {
-        int rc = h->precision == HYOWON_FP32_FIXED ? fp32::sort_current(h->f32, h->stream, h->d_status)
-                                                   : sort_current(h);
-        if (rc) return h->precision == HYOWON_FP32_FIXED ? status_or_cuda(h, rc) : rc;
+    bool sorted_here = false;
+    if (!h->sorted && h->precision == HYOWON_FP32_FIXED) {
+        int rc = fp32::sort_current(h->f32, h->stream, h->d_status);
+        if (rc) return status_or_cuda(h, rc);
         h->sorted = true;
     }
-    if (h->precision == HYOWON_FP64 && h->order_state == 0) {
+    if (h->sorted && h->precision == HYOWON_FP64 && h->order_state == 0) {
         int rc = index_current(h);
         if (rc) return rc;
     }
     CK(cudaMemsetAsync(h->d_status, 0, sizeof(unsigned int), h->stream));
+    if (!h->sorted) {
+        int rc = sort_current(h, true);
+        if (rc) return rc;
+        sorted_here = true;
+    }
     record(h, 0);
     int rc = enqueue_force(h, h->pc, h->mc, false, 0.0, current_order(h));
     if (rc) return rc;
@@ -617,6 +632,11 @@ int solve_force(hyowon_pm_t h) {
     rc = read_status(h, &st);
     if (rc) return rc;
     collect_timing(h);
+    if (sorted_here && (st & ST_BLOCKS_PUBLISH)) {
+        swap_sets(h);   // nothing was permuted
+        h->sorted = false;
+        h->order_state = 0;
+    }
     if (st) {
         h->acc_valid = false;
         return status_to_code(h, st);
@@ -1000,17 +1020,15 @@ int hyowon_pm_upload(hyowon_pm_t h, uint64_t n64, const double* x, const double*
     for (int a = 0; a < 3; ++a) {
         if (moms[a]) {
             CK(cudaMemcpyAsync(h->mom[0][a], moms[a], sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
-        } else {
-            CK(cudaMemsetAsync(h->mom[0][a], 0, sizeof(double) * n, h->stream));
         }
     }
     if (masses) CK(cudaMemcpyAsync(h->mass[0], masses, sizeof(double) * n, cudaMemcpyHostToDevice, h->stream));
-    ++h->launches;
-    launch_iota_u32(n, h->id[0], h->stream);
     CK(cudaMemsetAsync(h->d_status, 0, sizeof(unsigned int), h->stream));
     ++h->launches;
-    launch_validate_inputs_f64(n, h->pos[0][0], h->pos[0][1], h->pos[0][2],
-                               masses ? h->mass[0] : nullptr, h->d_status, h->stream);
+    launch_accept_upload_f64(n, h->pos[0][0], h->pos[0][1], h->pos[0][2],
+                             masses ? h->mass[0] : nullptr, h->id[0], px ? nullptr : h->mom[0][0],
+                             py ? nullptr : h->mom[0][1], pz ? nullptr : h->mom[0][2], h->d_status,
+                             h->stream);
     unsigned int st = 0;
     rc = read_status(h, &st);
     if (rc) return rc;
@@ -1186,6 +1204,41 @@ int hyowon_pm_download(hyowon_pm_t h, double* x, double* y, double* z, double* p
         return status_or_cuda(h, rc);
     }
     const uint32_t n = h->n;
+    // Up to 262,144 particles (2 MB a component) the calls cost more than the
+    // copies: every component is put in the caller's order by one kernel (six at a
+    // time, in the spare buffers) and copied on the handle's stream.
+    if (n <= 262144u) {
+        double* const spare[6] = {h->pos[1 - h->pc][0], h->pos[1 - h->pc][1], h->pos[1 - h->pc][2],
+                                  h->mom[1 - h->mc][0], h->mom[1 - h->mc][1], h->mom[1 - h->mc][2]};
+        const double* from[6];
+        double* to[6];
+        int k = 0;
+        auto send = [&]() {
+            if (k == 0) return cudaSuccess;
+            ++h->launches;
+            launch_unpermute_multi_f64(n, h->id[h->ic], k, from, spare, h->stream);
+            for (int c = 0; c < k; ++c) {
+                const cudaError_t e = cudaMemcpyAsync(to[c], spare[c], sizeof(double) * n,
+                                                      cudaMemcpyDeviceToHost, h->stream);
+                if (e != cudaSuccess) return e;
+            }
+            k = 0;
+            return cudaSuccess;
+        };
+        double* const host[9] = {x, y, z, px, py, pz, ax, ay, az};
+        const double* const dev[9] = {h->pos[h->pc][0], h->pos[h->pc][1], h->pos[h->pc][2],
+                                      h->mom[h->mc][0], h->mom[h->mc][1], h->mom[h->mc][2],
+                                      h->acc[0], h->acc[1], h->acc[2]};
+        for (int a = 0; a < 9; ++a) {
+            if (!host[a]) continue;
+            from[k] = dev[a];
+            to[k++] = host[a];
+            if (k == 6) CK(send());
+        }
+        CK(send());
+        CK(cudaStreamSynchronize(h->stream));
+        return HYOWON_OK;
+    }
     // The spare position buffers are dead between calls: two of them stage
     // the reordered components, so that the reorder of one component on the
     // handle's stream overlaps the device-to-host copy of the previous one on

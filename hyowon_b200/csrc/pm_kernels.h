@@ -42,6 +42,9 @@ void launch_scatter_f64(uint32_t n, const uint32_t* key, const uint32_t* rank,
                         const unsigned int* status, cudaStream_t s);
 void launch_unpermute_f64(uint32_t n, const uint32_t* id, const double* src, double* dst,
                           cudaStream_t s);
+// Up to eight arrays at once: dst[a][id[i]] = src[a][i].
+void launch_unpermute_multi_f64(uint32_t n, const uint32_t* id, int count,
+                                const double* const* src, double* const* dst, cudaStream_t s);
 void launch_scatter_multi(uint32_t n, const uint32_t* key, const uint32_t* rank,
                           const uint32_t* offset, int n_f64, const double* const* src,
                           double* const* dst, int n_u32, const uint32_t* const* src_u,
@@ -56,9 +59,11 @@ void launch_order(uint32_t n, const uint32_t* key, const uint32_t* rank, const u
                   uint32_t* order, const unsigned int* status, cudaStream_t s);
 
 // ---- FP64 form (pm_fp64.cu) -----------------------------------------------
-void launch_validate_inputs_f64(uint32_t n, const double* x, const double* y,
-                                const double* z, const double* mass, unsigned int* status,
-                                cudaStream_t s);
+// Checks an uploaded set, writes ids 0 .. n-1 and zeroes the momentum components
+// that are non-null.
+void launch_accept_upload_f64(uint32_t n, const double* x, const double* y, const double* z,
+                              const double* mass, uint32_t* id, double* px, double* py, double* pz,
+                              unsigned int* status, cudaStream_t s);
 void launch_key_f64(uint32_t n, const ParticlesF64& p, Axis a, const SortWork& w,
                     unsigned int* status, cudaStream_t s);
 void launch_kick_drift_key_f64(uint32_t n, const ParticlesF64& cur, const double* ax,

@@ -167,6 +167,16 @@ __global__ void k_unpermute(uint32_t n, const uint32_t* __restrict__ id,
     dst[id[i]] = src[i];
 }
 
+__global__ void k_unpermute_multi(uint32_t n, const uint32_t* __restrict__ id, ScatterArrays arr) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const uint32_t d = id[i];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) {
+        if (a < arr.n_f64) arr.dst[a][d] = arr.src[a][i];
+    }
+}
+
 // Cell order of the particles without moving them: order[offset[key]+rank] = i.
 __global__ void k_order(uint32_t n, const uint32_t* __restrict__ key,
                         const uint32_t* __restrict__ rank, const uint32_t* __restrict__ offset,
@@ -269,6 +279,18 @@ void launch_unpermute_f64(uint32_t n, const uint32_t* id, const double* src, dou
                           cudaStream_t s) {
     if (n == 0) return;
     k_unpermute<<<blocks_for(n, 256), 256, 0, s>>>(n, id, src, dst);
+}
+
+void launch_unpermute_multi_f64(uint32_t n, const uint32_t* id, int count,
+                                const double* const* src, double* const* dst, cudaStream_t s) {
+    if (n == 0) return;
+    ScatterArrays a{};
+    for (int i = 0; i < count; ++i) {
+        a.src[i] = src[i];
+        a.dst[i] = dst[i];
+    }
+    a.n_f64 = count;
+    k_unpermute_multi<<<blocks_for(n, 256), 256, 0, s>>>(n, id, a);
 }
 
 void launch_order(uint32_t n, const uint32_t* key, const uint32_t* rank, const uint32_t* offset,
