@@ -58,7 +58,7 @@ def reference_root(ref_root: str | None = None) -> str:
 def build_reference(ref_root: str | None = None) -> bool:
     """Compile the reference's hot path into oracle/_ref when its tree exists."""
     root = reference_root(ref_root)
-    if not root or not os.path.isdir(root):
+    if not root or not os.path.isdir(os.path.join(root, "src")):
         return os.path.exists(REF_SO)
     jobs = str(max(1, min(16, os.cpu_count() or 1)))
     subprocess.run(["make", "-s", f"-j{jobs}", "-C", os.path.join(HERE, "ref"),
