@@ -1,10 +1,12 @@
-// pm_tree.cu -- TreePM short-range force: Morton-key octree + warp-cooperative
+// pm_tree.cu -- TreePM short-range force: Hilbert-ordered octree + warp-cooperative
 // walk (include/hyowon_treepm.h).
 //
 // Build:
-//   1. 63-bit Morton key per source (21 bits per axis, x most significant, so
-//      the octant of a level-l node is bits 3(21-l)..3(21-l)+2 with x >= centre
-//      as bit 2, the reference's octant order, src/gravity/octree.cpp:336-357);
+//   1. 63-bit Hilbert index per source (21 bits per axis). Its leading 3 l bits are
+//      those of the level-l octree cell, so a cell's sources are consecutive, as
+//      they are in the reference's octant order (src/gravity/octree.cpp:336-357),
+//      and neighbours along the curve share a face at every level: a group of
+//      consecutive targets has a box a fifth smaller per side than in Morton order;
 //   2. stable LSD radix sort of (key, index), 8 passes of 8 bits;
 //   3. node extraction in one sweep: a node at level l is a maximal run of equal
 //      key >> 3(21-l) whose parent run holds >= 2 sources; runs holding one
@@ -80,6 +82,39 @@ __device__ __forceinline__ unsigned quant(double w, double L) {
     return static_cast<unsigned>(t);
 }
 
+// Hilbert index of a cell of the 2^21 lattice, by the bitwise transform of
+// J. Skilling, "Programming the Hilbert curve", AIP Conf. Proc. 707, 381 (2004): the
+// axes' bits are exchanged or inverted below each set or cleared bit from the top
+// down, then Gray-coded; bit triples read in order give the index.
+__device__ __forceinline__ unsigned long long hilbert_key(unsigned x, unsigned y, unsigned z) {
+#pragma unroll 1
+    for (unsigned q = 1u << (kBits - 1); q > 1u; q >>= 1) {
+        const unsigned low = q - 1u;
+        if (x & q) x ^= low;
+        unsigned t = (x ^ y) & low;
+        if (y & q) {
+            x ^= low;
+        } else {
+            x ^= t;
+            y ^= t;
+        }
+        t = (x ^ z) & low;
+        if (z & q) {
+            x ^= low;
+        } else {
+            x ^= t;
+            z ^= t;
+        }
+    }
+    y ^= x;
+    z ^= y;
+    unsigned t = 0;
+#pragma unroll 1
+    for (unsigned q = 1u << (kBits - 1); q > 1u; q >>= 1)
+        if (z & q) t ^= q - 1u;
+    return (spread3(x ^ t) << 2) | (spread3(y ^ t) << 1) | spread3(z ^ t);
+}
+
 __global__ void k_keys(uint32_t n, const double* __restrict__ x, const double* __restrict__ y,
                        const double* __restrict__ z, double L, double* __restrict__ wx,
                        double* __restrict__ wy, double* __restrict__ wz,
@@ -94,7 +129,7 @@ __global__ void k_keys(uint32_t n, const double* __restrict__ x, const double* _
     wx[i] = a;
     wy[i] = b;
     wz[i] = c;
-    key[i] = (spread3(quant(a, L)) << 2) | (spread3(quant(b, L)) << 1) | spread3(quant(c, L));
+    key[i] = hilbert_key(quant(a, L), quant(b, L), quant(c, L));
     val[i] = i;
 }
 
@@ -286,7 +321,8 @@ __device__ __forceinline__ uint32_t run_end(uint32_t n, const unsigned long long
 // and 18.4 -> 9.1 for 16.8M.
 __global__ void __launch_bounds__(kT)
 k_emit_nodes(uint32_t n, const unsigned long long* __restrict__ key, uint32_t n_tiles,
-             const uint32_t* __restrict__ offs, double L,
+             const uint32_t* __restrict__ offs, double L, const double* __restrict__ sx,
+             const double* __restrict__ sy, const double* __restrict__ sz,
              const unsigned long long* __restrict__ qx, const unsigned long long* __restrict__ qy,
              const unsigned long long* __restrict__ qz, double m, Node* __restrict__ nodes) {
     __shared__ uint32_t base[kT / 32][kLevels];   // first number of each warp's nodes
@@ -313,6 +349,8 @@ k_emit_nodes(uint32_t n, const unsigned long long* __restrict__ key, uint32_t n_
     }
     __syncthreads();
     const unsigned long long k = i < n ? key[i] : 0ull;
+    const unsigned ux = i < n ? quant(sx[i], L) : 0u, uy = i < n ? quant(sy[i], L) : 0u,
+                   uz = i < n ? quant(sz[i], L) : 0u;
     uint32_t child = 0xffffffffu, end = i + 1;
     for (int l = last; l >= first; --l) {
         const bool mine = l >= lo && l <= hi;
@@ -325,14 +363,8 @@ k_emit_nodes(uint32_t n, const unsigned long long* __restrict__ key, uint32_t n_
         if (l <= next) end = run_end(n, key, nd.prefix, shift, end - 1);
         const uint32_t cnt = end - i;
         nd.leaf = (cnt == 1 || l == kBits) ? 1u : 0u;
-        // cube: integer coordinates of the level-l cell from the prefix bits
-        unsigned cxi = 0, cyi = 0, czi = 0;
-        for (int d = l - 1; d >= 0; --d) {
-            const unsigned o = static_cast<unsigned>(nd.prefix >> (3 * d)) & 7u;
-            cxi = (cxi << 1) | (o >> 2);
-            cyi = (cyi << 1) | ((o >> 1) & 1u);
-            czi = (czi << 1) | (o & 1u);
-        }
+        // cube: the level-l cell of the source's lattice coordinates
+        const unsigned cxi = ux >> (kBits - l), cyi = uy >> (kBits - l), czi = uz >> (kBits - l);
         const double side = L / static_cast<double>(1ull << l);
         nd.half = 0.5 * side;
         nd.cx = (cxi + 0.5) * side;
@@ -1165,11 +1197,12 @@ void launch_walk(const WalkArgs& A, int group, cudaStream_t s) {
 // Targets a warp takes. A larger group shares the node tests among more targets
 // but has a larger box, so more undecided nodes and rejected pairs, and fewer
 // warps. Measured walk ms at G = 4 / 8 / 16 (clustered sources, every source a
-// target): 30,000: 1.0 / 1.5 / 2.3; 262,144: 6.5 / 4.9 / 6.4; 2.1M: 48 / 36 / 32;
-// 16.8M: 357 / 249 / 191 (one lane per target: 15, 48, 168 and 696). Targets that
-// are a sample of the sources lie further apart: of 2.1M sources, 4,096 targets
-// take 0.7 ms at G = 1 (12 at 4; 48 with one lane per target), 131,072 6.2 (9.8),
-// 524,288 23 at G = 1, 17 at 4, 15 at 8 and 25 at 16 (82).
+// target): 30,000: 0.87 / 0.96 / 1.36; 262,144: 4.7 / 4.0 / 4.9; 2.1M: 39 / 30 / 25;
+// 16.8M: 290 / 213 / 166 (in Morton order 25 to 30% more: 4.9, 32 and 191 at the
+// chosen G; one lane per target: 15, 48, 168 and 696). Targets that are a sample of
+// the sources lie further apart: of 2.1M sources, 4,096 targets take 0.66 ms at
+// G = 1 (1.6 at 4; 48 with one lane per target), 524,288 12 at G = 4, 10.4 at 8 and
+// 10.3 at 16 (23 at 1, 82 with one lane per target).
 int walk_group(uint32_t n, uint32_t nt) {
     if (nt < n / 8 + 1) return 1;
     if (nt < 100000) return 4;
@@ -1258,8 +1291,8 @@ int run(const hyowon_treepm_params& P, uint32_t n, const double* x, const double
     for (int l = 1; l < kLevels; ++l)
         if (level_begin[l + 1] > level_begin[l]) depth = l;
     Node* nodes = mem.get<Node>(node_base);
-    k_emit_nodes<<<n_node_tiles, kT, 0, s>>>(n, skey, n_node_tiles, level_offs, P.box_size, pq[0],
-                                             pq[1], pq[2], P.particle_mass, nodes);
+    k_emit_nodes<<<n_node_tiles, kT, 0, s>>>(n, skey, n_node_tiles, level_offs, P.box_size, sx, sy,
+                                             sz, pq[0], pq[1], pq[2], P.particle_mass, nodes);
     if (sm) {
         for (int l = depth; l >= 0; --l) {
             const uint32_t b = level_begin[l], e = level_begin[l + 1];

@@ -12,9 +12,9 @@
  * criterion r > l/theta + |COM - centre|_1 when the node neither contains the
  * target nor straddles the cutoff sphere (src/gravity/tree_walk.cpp:75-126,
  * 203-464). The octree covers [0, L)^3 and subdivides until one source per leaf
- * (src/gravity/octree.cpp:169-440); here it is built from 63-bit Morton keys
- * (21 bits per axis, x most significant), so coincident sources at that
- * resolution share an exact-pair leaf.
+ * (src/gravity/octree.cpp:169-440); here it is built from 63-bit Hilbert
+ * indices (21 bits per axis), so coincident sources at that resolution share an
+ * exact-pair leaf.
  */
 #ifndef HYOWON_TREEPM_H
 #define HYOWON_TREEPM_H
