@@ -573,14 +573,6 @@ struct Fail {
         if ((call) != CUFFT_SUCCESS) throw Fail{6, std::string(#call)};       \
     } while (0)
 
-template <typename T>
-T* dmalloc(size_t count, std::vector<void*>& owned) {
-    void* p = nullptr;
-    ACK(cudaMalloc(&p, (count ? count : 1) * sizeof(T)));
-    owned.push_back(p);
-    return static_cast<T*>(p);
-}
-
 // One device block that a run's work arrays are carved from (256-byte aligned),
 // kept between the runs of an engine: some sixty cudaMalloc / cudaFree pairs a
 // call took four fifths of a 128^3 gradient's 55 ms.
@@ -628,6 +620,22 @@ private:
     size_t cap_ = 0, off_ = 0;
 };
 
+struct PlanHandle {
+    cufftHandle h = 0;
+    bool made = false;
+    cufftResult create() {
+        const cufftResult r = cufftCreate(&h);
+        made = r == CUFFT_SUCCESS;
+        return r;
+    }
+    PlanHandle() = default;
+    PlanHandle(const PlanHandle&) = delete;
+    PlanHandle& operator=(const PlanHandle&) = delete;
+    ~PlanHandle() {
+        if (made) cufftDestroy(h);
+    }
+};
+
 struct Events {
     cudaEvent_t e[3] = {};
     Events() { for (auto& v : e) cudaEventCreate(&v); }
@@ -661,17 +669,43 @@ public:
             const double sn = std::sin(pi * static_cast<double>(mode) / N_);
             lap[i] = static_cast<R>(-4.0 / (dx * dx) * sn * sn);
         }
-        lap_ = dmalloc<R>(N_, owned_);
-        ACK(cudaMemcpy(lap_, lap.data(), sizeof(R) * N_, cudaMemcpyHostToDevice));
         four_pi_G_ = 4.0 * pi * G;
         scale_ = 1.0 / (dx * dx * dx) / static_cast<double>(cells_);
         five_ = poisson::supported(N_);
+        size_t fft_bytes = 0, modes = half_;
+        if (five_) {
+            modes = sizeof(R) == 8 ? poisson::modes_elements_f64(N_) : poisson::modes_elements_f32(N_);
+        } else {
+            AFFT(r2c_.create());
+            AFFT(c2r_.create());
+            cufftSetAutoAllocation(r2c_.h, 0);
+            cufftSetAutoAllocation(c2r_.h, 0);
+            size_t w1 = 0, w2 = 0;
+            AFFT(cufftMakePlan3d(r2c_.h, N_, N_, N_, FFTTypes<R>::R2C, &w1));
+            AFFT(cufftMakePlan3d(c2r_.h, N_, N_, N_, FFTTypes<R>::C2R, &w2));
+            fft_bytes = w1 > w2 ? w1 : w2;
+        }
+        char* ws = nullptr;
+        fixed_.plan([&] {
+            lap_ = fixed_.template take<R>(N_);
+            tw_ = fixed_.template take<C>(N_);
+            c_green_dev_ = fixed_.template take<R>(1);
+            status_ = fixed_.template take<unsigned int>(1);
+            ws = fixed_.template take<char>(fft_bytes);
+            modes_ = fixed_.template take<C>(modes);
+            mesh_ = fixed_.template take<R>(cells_);
+            phi_own_ = fixed_.template take<R>(cells_);
+            for (int a = 0; a < 3; ++a) {
+                x_[a] = fixed_.template take<double>(n_);
+                p_[a] = fixed_.template take<R>(n_);
+                acc_[a] = fixed_.template take<R>(n_);
+            }
+        });
+        phi_ = phi_own_;
+        ACK(cudaMemcpy(lap_, lap.data(), sizeof(R) * N_, cudaMemcpyHostToDevice));
         if (five_) {
             // the production five-pass solve: own transforms with the Green's
             // multiply fused into the x pass (chunked half spectrum)
-            const size_t elems = sizeof(R) == 8 ? poisson::modes_elements_f64(N_)
-                                                : poisson::modes_elements_f32(N_);
-            modes_ = dmalloc<C>(elems, owned_);
             const char* perr = nullptr;
             plan_ = poisson::create_plan(N_, sizeof(R) == 4, modes_, &perr);
             if (!plan_) throw Fail{HYOWON_ECUDA, perr ? perr : "five-pass plan"};
@@ -682,35 +716,13 @@ public:
                 tc[i].x = static_cast<R>(t[2 * i]);
                 tc[i].y = static_cast<R>(t[2 * i + 1]);
             }
-            tw_ = dmalloc<C>(N_, owned_);
             ACK(cudaMemcpy(tw_, tc.data(), sizeof(C) * N_, cudaMemcpyHostToDevice));
-            c_green_dev_ = dmalloc<R>(1, owned_);
             ACK(cudaMemcpy(c_green_dev_, &c_green_, sizeof(R), cudaMemcpyHostToDevice));
         } else {
-            AFFT(cufftCreate(&r2c_));
-            AFFT(cufftCreate(&c2r_));
-            plans_ = true;
-            cufftSetAutoAllocation(r2c_, 0);
-            cufftSetAutoAllocation(c2r_, 0);
-            size_t w1 = 0, w2 = 0;
-            AFFT(cufftMakePlan3d(r2c_, N_, N_, N_, FFTTypes<R>::R2C, &w1));
-            AFFT(cufftMakePlan3d(c2r_, N_, N_, N_, FFTTypes<R>::C2R, &w2));
-            void* ws = dmalloc<char>(w1 > w2 ? w1 : w2, owned_);
-            cufftSetWorkArea(r2c_, ws);
-            cufftSetWorkArea(c2r_, ws);
-            cufftSetStream(r2c_, s_);
-            cufftSetStream(c2r_, s_);
-            modes_ = dmalloc<C>(half_, owned_);
-        }
-        mesh_ = dmalloc<R>(cells_, owned_);
-        phi_own_ = dmalloc<R>(cells_, owned_);
-        phi_ = phi_own_;
-        status_ = dmalloc<unsigned int>(1, owned_);
-        ACK(cudaMemsetAsync(status_, 0, sizeof(unsigned int), s_));
-        for (int a = 0; a < 3; ++a) {
-            x_[a] = dmalloc<double>(n_, owned_);
-            p_[a] = dmalloc<R>(n_, owned_);
-            acc_[a] = dmalloc<R>(n_, owned_);
+            cufftSetWorkArea(r2c_.h, ws);
+            cufftSetWorkArea(c2r_.h, ws);
+            cufftSetStream(r2c_.h, s_);
+            cufftSetStream(c2r_.h, s_);
         }
     }
 
@@ -732,11 +744,6 @@ public:
 
     ~Engine() {
         poisson::destroy_plan(plan_);
-        if (plans_) {
-            cufftDestroy(r2c_);
-            cufftDestroy(c2r_);
-        }
-        for (void* p : owned_) cudaFree(p);
     }
 
     // acc = F(x); phi_ = potential at x, in the engine's own mesh.
@@ -774,9 +781,9 @@ public:
             if (k) throw Fail{HYOWON_ECUDA, "potential solve launch failed"};
             return;
         }
-        AFFT(FFTTypes<R>::fwd(r2c_, in, modes_));
+        AFFT(FFTTypes<R>::fwd(r2c_.h, in, modes_));
         k_green<R, C><<<nb(half_), kT, 0, s_>>>(N_, modes_, lap_, c_green_);
-        AFFT(FFTTypes<R>::inv(c2r_, modes_, out));
+        AFFT(FFTTypes<R>::inv(c2r_.h, modes_, out));
     }
 
     void kick(double K) {
@@ -1013,13 +1020,12 @@ private:
     Axis axis_{};
     R inv_two_dx_ = 0, c_green_ = 0;
     R* lap_ = nullptr;
-    cufftHandle r2c_ = 0, c2r_ = 0;
+    PlanHandle r2c_, c2r_;
     bool five_ = false;               // power-of-two mesh: five-pass solve
     poisson::Plan* plan_ = nullptr;
     C* tw_ = nullptr;
     R* c_green_dev_ = nullptr;
     double four_pi_G_ = 0.0, scale_ = 0.0;
-    bool plans_ = false;
     R* mesh_ = nullptr;
     R* phi_own_ = nullptr;
     R* phi_ = nullptr;
@@ -1029,7 +1035,7 @@ private:
     R* p_[3] = {};
     R* acc_[3] = {};
     uint64_t solves_ = 0, vjps_ = 0;
-    std::vector<void*> owned_;
+    Arena fixed_;       // what the engine keeps: meshes, spectrum, particle state
     Arena arena_;       // a run's work arrays
     LptWork lpt_;
 };

@@ -167,13 +167,6 @@ int LptWork::require(int n_side, cudaStream_t s, const char** err) {
         const size_t cells = static_cast<size_t>(n_side) * n_side * n_side;
         const size_t half = static_cast<size_t>(n_side) * n_side * (n_side / 2 + 1);
         size_t w1 = 0, w2 = 0;
-        if (cudaMalloc(&delta, sizeof(double2) * half) != cudaSuccess
-            || cudaMalloc(&work, sizeof(double2) * half) != cudaSuccess
-            || cudaMalloc(&real, sizeof(double) * cells) != cudaSuccess) {
-            *err = "LPT work arrays could not be allocated";
-            release();
-            return 7;
-        }
         if (cufftCreate(&r2c) != CUFFT_SUCCESS) {
             *err = "cufftCreate failed";
             release();
@@ -194,13 +187,19 @@ int LptWork::require(int n_side, cudaStream_t s, const char** err) {
             release();
             return 6;
         }
-        if (cudaMalloc(&fft, w1 > w2 ? w1 : w2) != cudaSuccess) {
-            *err = "cuFFT workspace could not be allocated";
+        const size_t spectrum = (sizeof(double2) * half + 255) & ~static_cast<size_t>(255);
+        const size_t mesh = (sizeof(double) * cells + 255) & ~static_cast<size_t>(255);
+        if (cudaMalloc(&block, 2 * spectrum + mesh + (w1 > w2 ? w1 : w2)) != cudaSuccess) {
+            *err = "LPT work arrays could not be allocated";
             release();
             return 7;
         }
-        cufftSetWorkArea(r2c, fft);
-        cufftSetWorkArea(c2r, fft);
+        char* at = static_cast<char*>(block);
+        delta = reinterpret_cast<double2*>(at);
+        work = reinterpret_cast<double2*>(at + spectrum);
+        real = reinterpret_cast<double*>(at + 2 * spectrum);
+        cufftSetWorkArea(r2c, at + 2 * spectrum + mesh);
+        cufftSetWorkArea(c2r, at + 2 * spectrum + mesh);
         N = n_side;
     }
     cufftSetStream(r2c, s);
@@ -214,11 +213,8 @@ void LptWork::release() {
         cufftDestroy(c2r);
     }
     plans = false;
-    cudaFree(fft);
-    cudaFree(delta);
-    cudaFree(work);
-    cudaFree(real);
-    fft = nullptr;
+    cudaFree(block);
+    block = nullptr;
     delta = work = nullptr;
     real = nullptr;
     N = 0;

@@ -9,10 +9,10 @@ namespace hyowon {
 // side; made on first use, freed with the object (or by release()).
 struct LptWork {
     int N = 0;
+    void* block = nullptr;      // one allocation: the arrays below and cuFFT's own
     double2* delta = nullptr;   // half spectra
     double2* work = nullptr;
     double* real = nullptr;
-    void* fft = nullptr;
     int r2c = 0, c2r = 0;       // cufftHandle
     bool plans = false;
     // 0, 6 (CUDA / cuFFT) or 7 (allocation); *err names the failure.
