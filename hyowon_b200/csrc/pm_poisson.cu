@@ -25,6 +25,7 @@
 
 #include <cuda.h>
 
+#include <atomic>
 #include <cmath>
 #include <new>
 
@@ -155,7 +156,11 @@ template <typename T, int LOG2N, int MODE> struct ColumnCfg {
     static constexpr int nbuf = single_buffer ? 1 : G::nbuf_b;
     static constexpr size_t smem = static_cast<size_t>(nbuf) * G::tile_bytes_b;
     static constexpr int smem_blocks = static_cast<int>((227u * 1024u) / smem);
-    static constexpr int want = LOG2N >= 10 ? 2 : 3;
+    // Small meshes have small blocks (64 threads at N = 256 in binary64): as many
+    // per SM as make 512 (FP32 768) threads. At 256^3 the binary64 x pass then takes
+    // 82 us instead of 108 at three blocks of 64 threads (85 at 384 threads).
+    static constexpr int fill = (sizeof(T) == 8 ? 512 : 768) / G::TCB;
+    static constexpr int want = LOG2N >= 10 ? 2 : (LOG2N == 9 ? 3 : (fill < 16 ? fill : 16));
     static constexpr int minb =
         single_buffer ? G::SP * (want < smem_blocks ? want : smem_blocks) : G::minb_c;
 };
@@ -513,17 +518,36 @@ k_columns(const __grid_constant__ CUtensorMap map, cx_t<T>* __restrict__ H,
     }
 }
 
-template <typename K>
-bool prepare(K kernel, size_t smem) {
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                static_cast<int>(smem)) == cudaSuccess;
+// Resident blocks of a kernel on the whole device, its dynamic shared memory
+// allowed; worked out once per kernel and device (five runtime calls, some 5 us,
+// that every launch made). 0 on failure.
+template <auto KERNEL>
+unsigned resident_blocks(int threads, size_t smem) {
+    static std::atomic<unsigned> known[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    const bool slot = dev >= 0 && dev < 64;
+    if (slot) {
+        const unsigned k = known[dev].load(std::memory_order_acquire);
+        if (k) return k;
+    }
+    int sms = 0, per_sm = 0;
+    if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(smem)) != cudaSuccess
+        || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess
+        || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, KERNEL, threads, smem) != cudaSuccess
+        || per_sm < 1)
+        return 0;
+    const unsigned full = static_cast<unsigned>(sms) * static_cast<unsigned>(per_sm);
+    if (slot) known[dev].store(full, std::memory_order_release);
+    return full;
 }
 
 template <typename T, typename SRC, int LOG2N>
 int z_forward(const SRC* in, cx_t<T>* H, const cx_t<T>* tw, unsigned long long* qsum,
               cudaStream_t s) {
     using G = Geo<T, LOG2N>;
-    if (!prepare(k_z_forward<T, SRC, LOG2N>, G::smem_zf)) return -1;
+    if (!resident_blocks<k_z_forward<T, SRC, LOG2N>>(G::TZ, G::smem_zf)) return -1;
     const unsigned blocks = static_cast<unsigned>(static_cast<size_t>(G::N) * G::N / G::CZ);
     k_z_forward<T, SRC, LOG2N><<<blocks, G::TZ, G::smem_zf, s>>>(in, H, tw, qsum);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
@@ -532,7 +556,7 @@ int z_forward(const SRC* in, cx_t<T>* H, const cx_t<T>* tw, unsigned long long* 
 template <typename T, int LOG2N, typename EPI = StorePair>
 int z_inverse(const cx_t<T>* H, T* out, const cx_t<T>* tw, cudaStream_t s, EPI epi = EPI{}) {
     using G = Geo<T, LOG2N>;
-    if (!prepare(k_z_inverse<T, LOG2N, EPI>, G::smem_zi)) return -1;
+    if (!resident_blocks<k_z_inverse<T, LOG2N, EPI>>(G::TZ, G::smem_zi)) return -1;
     const unsigned blocks = static_cast<unsigned>(static_cast<size_t>(G::N) * G::N / G::CZ);
     k_z_inverse<T, LOG2N, EPI><<<blocks, G::TZ, G::smem_zi, s>>>(H, out, tw, epi);
     return cudaPeekAtLastError() == cudaSuccess ? 1 : -1;
@@ -587,15 +611,9 @@ int columns(const Plan* p, cx_t<T>* H, const cx_t<T>* tw, GF green, unsigned int
     if (!p || p->N != G::N) return -1;
     auto kernel = k_columns<T, LOG2N, AXIS, SIGN, MODE, GF>;
     constexpr size_t smem = ColumnCfg<T, LOG2N, MODE>::smem;
-    if (!prepare(kernel, smem)) return -1;
-    int dev = 0, sms = 0, per_sm = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess
-        || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess
-        || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, G::TCB, smem) != cudaSuccess
-        || per_sm < 1)
-        return -1;
+    const unsigned full = resident_blocks<k_columns<T, LOG2N, AXIS, SIGN, MODE, GF>>(G::TCB, smem);
+    if (!full) return -1;
     const unsigned tiles = static_cast<unsigned>(G::KC) * G::N * G::SP;
-    const unsigned full = static_cast<unsigned>(sms) * static_cast<unsigned>(per_sm);
     const unsigned grid = tiles < full ? tiles : full;
     kernel<<<grid, G::TCB, smem, s>>>(AXIS == 1 ? p->y : p->x, H, tw, green, status,
                                           p->wait_limit);
