@@ -169,7 +169,10 @@ long double window_axis(double k, double dx) {
     return s * s;
 }
 
+// The arrays of one call, carved from one device block that also holds cuFFT's work
+// area: eleven allocations and frees a call took longer than its kernels.
 struct Buffers {
+    void* block = nullptr;
     double* rho = nullptr;
     double2* modes = nullptr;
     double2* shifted = nullptr;
@@ -180,27 +183,20 @@ struct Buffers {
     double* sums = nullptr;
     unsigned long long* count = nullptr;
     unsigned int* status = nullptr;
+    char* work = nullptr;
     cufftHandle plan = 0;
     bool has_plan = false;
+    size_t bytes = 0;
+    template <typename T>
+    void take(T** p, size_t n) {
+        *p = block ? reinterpret_cast<T*>(static_cast<char*>(block) + bytes) : nullptr;
+        bytes += (n * sizeof(T) + 255) & ~static_cast<size_t>(255);
+    }
     ~Buffers() {
-        cudaFree(rho);
-        cudaFree(modes);
-        cudaFree(shifted);
-        cudaFree(pos);
-        cudaFree(tables);
-        cudaFree(partial);
-        cudaFree(pcount);
-        cudaFree(sums);
-        cudaFree(count);
-        cudaFree(status);
         if (has_plan) cufftDestroy(plan);
+        cudaFree(block);
     }
 };
-
-template <typename T>
-bool dalloc(T** p, size_t count) {
-    return cudaMalloc(reinterpret_cast<void**>(p), (count ? count : 1) * sizeof(T)) == cudaSuccess;
-}
 
 }  // namespace
 
@@ -244,19 +240,35 @@ int compute(double L, int N, uint32_t n, const double* x, const double* y, const
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int blocks = sms * 4;
-    if (!dalloc(&buf.rho, cells) || !dalloc(&buf.modes, half) || !dalloc(&buf.tables, tab.size())
-        || !dalloc(&buf.partial, static_cast<size_t>(blocks) * nb * kFields)
-        || !dalloc(&buf.pcount, static_cast<size_t>(blocks) * nb)
-        || !dalloc(&buf.sums, static_cast<size_t>(nb) * kFields) || !dalloc(&buf.count, nb)
-        || !dalloc(&buf.status, 1)
-        || (req.interlaced && (!dalloc(&buf.shifted, half) || !dalloc(&buf.pos, 3ull * n))))
-        return fail(HYOWON_ENOMEM, "power spectrum: device allocation failed");
     if (cufftCreate(&buf.plan) != CUFFT_SUCCESS)
         return fail(HYOWON_ECUDA, "power spectrum: cuFFT plan creation failed");
     buf.has_plan = true;
     size_t work = 0;
-    if (cufftMakePlan3d(buf.plan, N, N, N, CUFFT_D2Z, &work) != CUFFT_SUCCESS
+    if (cufftSetAutoAllocation(buf.plan, 0) != CUFFT_SUCCESS
+        || cufftMakePlan3d(buf.plan, N, N, N, CUFFT_D2Z, &work) != CUFFT_SUCCESS
         || cufftSetStream(buf.plan, s) != CUFFT_SUCCESS)
+        return fail(HYOWON_ECUDA, "power spectrum: cuFFT plan creation failed");
+    auto layout = [&] {
+        buf.bytes = 0;
+        buf.take(&buf.rho, cells);
+        buf.take(&buf.modes, half);
+        buf.take(&buf.tables, tab.size());
+        buf.take(&buf.partial, static_cast<size_t>(blocks) * nb * kFields);
+        buf.take(&buf.pcount, static_cast<size_t>(blocks) * nb);
+        buf.take(&buf.sums, static_cast<size_t>(nb) * kFields);
+        buf.take(&buf.count, nb);
+        buf.take(&buf.status, 1);
+        if (req.interlaced) {
+            buf.take(&buf.shifted, half);
+            buf.take(&buf.pos, 3ull * n);
+        }
+        buf.take(&buf.work, work);
+    };
+    layout();
+    if (cudaMalloc(&buf.block, buf.bytes) != cudaSuccess)
+        return fail(HYOWON_ENOMEM, "power spectrum: device allocation failed");
+    layout();
+    if (cufftSetWorkArea(buf.plan, buf.work) != CUFFT_SUCCESS)
         return fail(HYOWON_ECUDA, "power spectrum: cuFFT plan creation failed");
     if (cudaMemcpyAsync(buf.tables, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice,
                         s) != cudaSuccess
