@@ -186,20 +186,21 @@ __global__ void k_scatter3(uint32_t n, const double* __restrict__ x, const doubl
         }
 }
 
-// s = sum_d (u_d[c+e_d] - u_d[c-e_d]) / (2 dx)
+// s = sum_d (u_d[c+e_d] - u_d[c-e_d]) / (2 dx); one block per row (y, x), so that no
+// thread divides a 64-bit cell number by N (18.6 us of a 128^3 mesh, whose four
+// arrays take 10).
 template <typename R>
 __global__ void k_divergence(int N, const R* __restrict__ u0, const R* __restrict__ u1,
                              const R* __restrict__ u2, R inv_two_dx, R* __restrict__ s) {
-    const uint64_t cells = static_cast<uint64_t>(N) * N * N;
-    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= cells) return;
-    const int z = static_cast<int>(i % N);
-    const int y = static_cast<int>((i / N) % N);
-    const int x = static_cast<int>(i / (static_cast<uint64_t>(N) * N));
-    s[i] = ((u0[cidx(up(x, N), y, z, N)] - u0[cidx(dn(x, N), y, z, N)])
-            + (u1[cidx(x, up(y, N), z, N)] - u1[cidx(x, dn(y, N), z, N)])
-            + (u2[cidx(x, y, up(z, N), N)] - u2[cidx(x, y, dn(z, N), N)]))
-        * inv_two_dx;
+    const int y = blockIdx.x, x = blockIdx.y;
+    const size_t row = cidx(x, y, 0, N);
+    const R* const xp = u0 + cidx(up(x, N), y, 0, N);
+    const R* const xm = u0 + cidx(dn(x, N), y, 0, N);
+    const R* const yp = u1 + cidx(x, up(y, N), 0, N);
+    const R* const ym = u1 + cidx(x, dn(y, N), 0, N);
+    const R* const zr = u2 + row;
+    for (int z = threadIdx.x; z < N; z += blockDim.x)
+        s[row + z] = ((xp[z] - xm[z]) + (yp[z] - ym[z]) + (zr[up(z, N)] - zr[dn(z, N)])) * inv_two_dx;
 }
 
 template <typename R, typename C>
@@ -797,10 +798,12 @@ public:
 
     // psi = A div(scatter(coef * lp)): the mesh half of VJP_F at x.
     void vjp_mesh(double coef, double* const lp[3], R* const u[3], R* psi) {
-        for (int a = 0; a < 3; ++a) ACK(cudaMemsetAsync(u[a], 0, sizeof(R) * cells_, s_));
+        // the three meshes lie one after the other
+        ACK(cudaMemsetAsync(u[0], 0, sizeof(R) * static_cast<size_t>(u[2] - u[0] + cells_), s_));
         k_scatter3<R><<<nb(n_), kT, 0, s_>>>(n_, x_[0], x_[1], x_[2], lp[0], lp[1], lp[2], coef, axis_,
                                              u[0], u[1], u[2]);
-        k_divergence<R><<<nb(cells_), kT, 0, s_>>>(N_, u[0], u[1], u[2], inv_two_dx_, mesh_);
+        const int row_threads = N_ >= kT ? kT : (N_ + 31) / 32 * 32;
+        k_divergence<R><<<dim3(N_, N_), row_threads, 0, s_>>>(N_, u[0], u[1], u[2], inv_two_dx_, mesh_);
         apply_green(mesh_, psi);
         ++vjps_;
     }
@@ -843,8 +846,8 @@ public:
                 for (int a = 0; a < 3; ++a) {
                     lx[a] = arena_.template take<double>(n_);
                     lp[a] = arena_.template take<double>(n_);
-                    u[a] = arena_.template take<R>(cells_);
                 }
+                for (int a = 0; a < 3; ++a) u[a] = arena_.template take<R>(cells_);
                 psi = arena_.template take<R>(cells_);
                 grad = arena_.template take<double>(n_);
             }

@@ -999,8 +999,8 @@ long double fit_poly(int deg, double t_max, double r_s, PairPoly* out) {
     out->tau = static_cast<double>(2.0L / (static_cast<long double>(t_max) * r_s * r_s));
     for (int k = 0; k < n; ++k) out->c[k] = static_cast<double>(mono[k] / rs3);
     long double worst = 0.0L;
-    for (int i = 0; i <= 400; ++i) {
-        const long double tau = -1.0L + 2.0L * i / 400.0L;
+    for (int i = 0; i <= 100; ++i) {
+        const long double tau = -1.0L + 2.0L * i / 100.0L;
         long double p = 0.0L;
         for (int k = deg; k >= 0; --k) p = p * tau + mono[k];
         const long double h = short_h(0.5L * t_max * (tau + 1.0L));
