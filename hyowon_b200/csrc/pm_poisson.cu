@@ -158,9 +158,10 @@ template <typename T, int LOG2N, int MODE> struct ColumnCfg {
     static constexpr int smem_blocks = static_cast<int>((227u * 1024u) / smem);
     // Small meshes have small blocks (64 threads at N = 256 in binary64): as many
     // per SM as make 512 (FP32 768) threads. At 256^3 the binary64 x pass then takes
-    // 82 us instead of 108 at three blocks of 64 threads (85 at 384 threads).
+    // 82 us instead of 108 at three blocks of 64 threads (85 at 384 threads), and at
+    // 512^3 700 us instead of 748 at three blocks of 128.
     static constexpr int fill = (sizeof(T) == 8 ? 512 : 768) / G::TCB;
-    static constexpr int want = LOG2N >= 10 ? 2 : (LOG2N == 9 ? 3 : (fill < 16 ? fill : 16));
+    static constexpr int want = LOG2N >= 10 ? 2 : (fill < 16 ? fill : 16);
     static constexpr int minb =
         single_buffer ? G::SP * (want < smem_blocks ? want : smem_blocks) : G::minb_c;
 };
