@@ -473,18 +473,66 @@ __global__ void k_walk_nodes(uint32_t n_nodes, double theta, double L, Node* __r
     gc[i] = make_uint4(nd.first_child, nd.n_child | (nd.leaf << 8), nd.start, nd.end - nd.start);
 }
 
-// The pair factor as A^3 - h, A = (r^2 + eps^2)^(-1/2), with the long-range part
-//   h(r^2) = (1 - M_S(q)) / r^3 = r_s^-3 sum_k (-1)^k q^(2k) 2(k+1) / ((2k+3) 4^(k+1) (k+1)! sqrt(pi)),
-// an entire function of t = q^2, as one polynomial in tau = 2 t / t_max - 1 over
-// the whole cutoff sphere (pair_poly, below): no branch, no error function, no
-// exponential. One rsqrt and DEG + 8 multiply-adds replace the erfc, exp, expm1,
+// The pair factor as A^3 F(u), A = (r^2 + eps^2)^(-1/2), u = 1/A, with
+//   F(u) = 1 - u^3 h(u^2 - eps^2),
+// h the long-range part (1 - M_S(q)) / r^3, an entire function of r^2: F is entire in
+// u, softening included, and one polynomial in v = b - k u serves the whole cutoff
+// sphere (v = 0 at the cutoff, 2 at r = 0; fit_poly, below): no branch, no error
+// function, no exponential. F falls to M_S(4.5) = 0.0175 and further, so a
+// polynomial for h, and A^3 - h formed from it, loses the outer pairs (5e-14 of them at
+// 4.5 r_s, 5e-12 at 6). Here the first two coefficients are those of the expansion
+// about the cutoff, where F is smallest, and the rest of the sum carries a factor v^2
+// there; u enters with its rounding error (amplified 9 times by F at 4.5 r_s)
+// restored. One rsqrt and DEG + 13 multiply-adds replace the erfc, exp, expm1,
 // log1p, sqrt and division of short_factor_impl, which remains for cutoffs of so
-// many r_s that no polynomial of these degrees reaches the accuracy (DEG = 0).
-constexpr int kDegLow = 12, kDegMid = 20, kDegHigh = 28;
+// many r_s, or softenings so large, that no polynomial of these degrees reaches its
+// accuracy (DEG = 0). Largest error of F over the sphere at 4.5 r_s: 1.0e-15 in
+// binary64 (the closed form 7e-16), 2.8e-8 in the precision form (FP32 closed form
+// 1.2e-6).
+//
+// The precision form takes A^3 - h, h of degree kDegFp32 in r^2, while that stays within
+// half an FP32 rounding of the factor (up to 4.5 r_s): seven operations fewer, 5% of a
+// walk of 16.8M sources.
+constexpr int kDegFp32 = 12, kDegLow = 22, kDegMid = 28, kDegHigh = 36;
 struct PairPoly {
-    double tau;                 // 2 / (t_max r_s^2)
-    double c[kDegHigh + 1];     // monomial coefficients in tau, times r_s^-3
+    double k, half_k, b;        // v = b - k u; degree kDegFp32: tau = k r^2 - 1
+    double c[kDegHigh + 1];     // c[0] + v (c[1] + v S(1 - v)), S's monomials from c[2];
+                                // degree kDegFp32: h's monomials in tau
 };
+
+// h at r^2.
+__host__ __device__ __forceinline__ double long_part(double r2, const PairPoly& pp) {
+    const double tau = fma(r2, pp.k, -1.0);
+    const double t2 = tau * tau;
+    double even = pp.c[kDegFp32], odd = pp.c[kDegFp32 - 1];
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (int k = kDegFp32 - 2; k >= 0; k -= 2) {
+        even = fma(even, t2, pp.c[k]);
+        if (k > 0) odd = fma(odd, t2, pp.c[k - 1]);
+    }
+    return fma(odd, tau, even);
+}
+
+// F at u = s a, s = r^2 + eps^2 and a its reciprocal square root.
+template <int DEG, bool EXACT_U>
+__host__ __device__ __forceinline__ double pair_poly(double s, double a, const PairPoly& pp) {
+    const double u = s * a;
+    double v = fma(-u, pp.k, pp.b);
+    if constexpr (EXACT_U) v = fma(-pp.half_k * a, fma(-u, u, s), v);
+    const double tau = 1.0 - v;
+    const double t2 = tau * tau;
+    double even = pp.c[DEG], odd = pp.c[DEG - 1];   // DEG is even
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (int k = DEG - 2; k >= 2; k -= 2) {
+        even = fma(even, t2, pp.c[k]);
+        if (k > 2) odd = fma(odd, t2, pp.c[k - 1]);
+    }
+    return fma(fma(fma(odd, tau, even), v, pp.c[1]), v, pp.c[0]);
+}
 
 template <typename R, int DEG>
 __device__ __forceinline__ double pair_factor(double r2, double eps2, double inv_rs,
@@ -494,14 +542,6 @@ __device__ __forceinline__ double pair_factor(double r2, double eps2, double inv
         return static_cast<double>(short_factor_impl<R>(static_cast<R>(r2), static_cast<R>(eps2),
                                                         irs, irs * irs * irs));
     } else {
-        const double tau = r2 * pp.tau - 1.0;
-        const double t2 = tau * tau;
-        double even = pp.c[DEG], odd = pp.c[DEG - 1];
-#pragma unroll
-        for (int k = DEG - 2; k >= 0; k -= 2) {
-            even = even * t2 + pp.c[k];
-            if (k > 0) odd = odd * t2 + pp.c[k - 1];
-        }
         const double s = r2 + eps2;
         double a;
         if constexpr (sizeof(R) == 8) {
@@ -511,7 +551,8 @@ __device__ __forceinline__ double pair_factor(double r2, double eps2, double inv
             a = static_cast<double>(rsqrtf(static_cast<float>(s)));
             a = a * (1.5 - 0.5 * s * a * a);
         }
-        return a * a * a - (odd * tau + even);
+        if constexpr (DEG == kDegFp32) return a * a * a - long_part(r2, pp);
+        else return a * a * a * pair_poly<DEG, sizeof(R) == 8>(s, a, pp);
     }
 }
 
@@ -956,57 +997,134 @@ k_walk(uint32_t n_targets, const uint32_t* __restrict__ tslot, const double* __r
     }
 }
 
-// Chebyshev interpolation of r_s^3 h over t in [0, t_max] at degree `deg`, in
-// monomials of tau; returns the largest dropped relative error seen on a fine
-// grid (relative to h, in long double).
-long double short_h(long double t) {
+// h r_s^3 at r^2 = t r_s^2, t <= 4: the alternating series, terms falling from the first.
+long double long_part_series(long double t) {
     const long double isp = 0.564189583547756286948079451560772586L;
-    if (t <= 4.0L) {   // the alternating series, terms falling from the first
-        long double term = 1.0L / 4.0L, sum = 0.0L;   // t^k / (4^(k+1) (k+1)!)
-        for (int k = 0; k < 40; ++k) {
-            sum += (k & 1 ? -term : term) * 2.0L * (k + 1) / (2 * k + 3);
-            term *= t / (4.0L * (k + 2));
-        }
-        return isp * sum;
+    long double term = 1.0L / 4.0L, sum = 0.0L;   // t^k / (4^(k+1) (k+1)!)
+    for (int k = 0; k < 30; ++k) {
+        sum += (k & 1 ? -term : term) * 2.0L * (k + 1) / (2 * k + 3);
+        term *= t / (4.0L * (k + 2));
     }
-    const long double q = std::sqrt(t);
-    return (std::erf(0.5L * q) - q * isp * std::exp(-0.25L * t)) / (t * q);
+    return isp * sum;
 }
 
-long double fit_poly(int deg, double t_max, double r_s, PairPoly* out) {
-    const int n = deg + 1;
-    const long double pi = 3.141592653589793238462643383279502884L;
-    std::vector<long double> cheb(n), mono(n, 0.0L), a(n, 0.0L), b(n, 0.0L);
-    std::vector<long double> y(n);
-    for (int k = 0; k < n; ++k)
-        y[k] = short_h(0.5L * t_max * (std::cos(pi * (k + 0.5L) / n) + 1.0L));
-    for (int j = 0; j < n; ++j) {
+long double shape_fraction(long double t) {   // M_S
+    const long double isp = 0.564189583547756286948079451560772586L, q = std::sqrt(t);
+    return std::erfc(0.5L * q) + q * isp * std::exp(-0.25L * t);
+}
+
+// F(u), the pair factor times s^(3/2), at r^2 = t r_s^2 and softening e r_s: below
+// t = 4 (M_S > 0.5) as 1 - u^3 h, beyond as in short_factor_impl, which keeps the
+// relative accuracy of a small F.
+long double pair_shape(long double t, long double e) {
+    const long double s = t + e * e, u3 = s * std::sqrt(s);
+    if (t <= 4.0L) return 1.0L - u3 * long_part_series(t);
+    return u3 / (t * std::sqrt(t)) * (std::expm1(-1.5L * std::log1p(e * e / t)) + shape_fraction(t));
+}
+
+constexpr long double kPiL = 3.141592653589793238462643383279502884L;
+
+// Chebyshev interpolation, in monomials of tau, of the values y[i] at the N nodes
+// tau_i = cos(pi (i + 1/2) / N).
+template <int N>
+void interpolate(const long double (&y)[N], long double (&mono)[N]) {
+    long double wave[4 * N], ta[N] = {}, tb[N] = {};
+    for (int i = 0; i < 4 * N; ++i) wave[i] = std::cos(kPiL * i / (2 * N));
+    for (int i = 0; i < N; ++i) mono[i] = 0.0L;
+    ta[0] = 1.0L;
+    tb[1] = 1.0L;
+    for (int j = 0; j < N; ++j) {
         long double s = 0.0L;
-        for (int k = 0; k < n; ++k) s += y[k] * std::cos(pi * j * (k + 0.5L) / n);
-        cheb[j] = s * (j ? 2.0L : 1.0L) / n;
+        for (int i = 0; i < N; ++i) s += y[i] * wave[j * (2 * i + 1) % (4 * N)];
+        s *= (j ? 2.0L : 1.0L) / N;
+        for (int i = 0; i < N; ++i) mono[i] += s * ta[i];
+        // T_j in monomials by the recurrence T_{j+1} = 2 tau T_j - T_{j-1}
+        for (int i = N - 1; i >= 0; --i) {
+            const long double old = tb[i];
+            tb[i] = (i ? 2.0L * tb[i - 1] : 0.0L) - ta[i];
+            ta[i] = old;
+        }
     }
-    // T_j in monomials by the recurrence T_{j+1} = 2 tau T_j - T_{j-1}
-    a[0] = 1.0L;
-    if (n > 1) b[1] = 1.0L;
-    for (int j = 0; j < n; ++j) {
-        for (int k = 0; k < n; ++k) mono[k] += cheb[j] * a[k];
-        std::vector<long double> c(n, 0.0L);
-        for (int k = 0; k < n; ++k) c[k] = (k ? 2.0L * b[k - 1] : 0.0L) - a[k];
-        a = b;
-        b = c;
+}
+
+// Whether the polynomial gives F within `want` of itself at 96 distances from the
+// cutoff inwards.
+template <int DEG, bool EXACT_U>
+bool close_to_shape(double ratio, double eps, double r_s, double want, const PairPoly& pp) {
+    for (int i = 0; i < 96; ++i) {
+        const double r = ratio * r_s * (1.0 - (i + 0.01) / 96.0);
+        const double r2 = r * r, s = r2 + eps * eps, root = std::sqrt(s);
+        const long double f = pair_shape(static_cast<long double>(r2) / r_s / r_s,
+                                         static_cast<long double>(eps) / r_s);
+        const long double p = DEG == kDegFp32 ? 1.0 - s * root * long_part(r2, pp)
+                                              : pair_poly<DEG, EXACT_U>(s, 1.0 / root, pp);
+        if (!(std::fabs(p - f) <= want * std::fabs(f))) return false;
     }
-    const long double rs3 = static_cast<long double>(r_s) * r_s * r_s;
-    out->tau = static_cast<double>(2.0L / (static_cast<long double>(t_max) * r_s * r_s));
-    for (int k = 0; k < n; ++k) out->c[k] = static_cast<double>(mono[k] / rs3);
-    long double worst = 0.0L;
-    for (int i = 0; i <= 100; ++i) {
-        const long double tau = -1.0L + 2.0L * i / 100.0L;
-        long double p = 0.0L;
-        for (int k = deg; k >= 0; --k) p = p * tau + mono[k];
-        const long double h = short_h(0.5L * t_max * (tau + 1.0L));
-        worst = std::max(worst, std::fabs(p - h) / h);
+    return true;
+}
+
+// The polynomial of degree DEG for a cutoff of `ratio` r_s: in v, two steps of division
+// by v taken off, or (degree kDegFp32) that of h; false when it is not within `want`.
+template <int DEG, bool EXACT_U>
+bool fit_poly(double ratio, double eps, double r_s, double want, PairPoly* out) {
+    constexpr int n = DEG + 1;
+    const long double e = static_cast<long double>(eps) / r_s;
+    const long double t_max = static_cast<long double>(ratio) * ratio * (1.0L + 1e-9L);
+    const long double u_max = std::sqrt(t_max + e * e), width = t_max / (u_max + e);
+    out->k = static_cast<double>(DEG == kDegFp32 ? 2.0L / (t_max * r_s * r_s) : 2.0L / (width * r_s));
+    out->half_k = 0.5 * out->k;
+    out->b = static_cast<double>(2.0L * u_max / width);
+    if (!std::isfinite(out->k) || !std::isfinite(out->b)) return false;
+    long double y[n], mono[n];
+    for (int i = 0; i < n; ++i) {
+        const long double tau = std::cos(kPiL * (i + 0.5L) / n);
+        if (DEG == kDegFp32) {
+            const long double t = 0.5L * t_max * (tau + 1.0L);
+            const long double h = t <= 4.0L ? long_part_series(t)
+                                            : (1.0L - shape_fraction(t)) / (t * std::sqrt(t));
+            y[i] = h / (static_cast<long double>(r_s) * r_s * r_s);
+        } else {   // u / r_s by the rounded k and b
+            const long double u = (static_cast<long double>(out->b) - 1.0L + tau)
+                / (static_cast<long double>(out->k) * r_s);
+            y[i] = pair_shape((u - e) * (u + e), e);
+        }
     }
-    return worst;
+    interpolate(y, mono);
+    for (int step = 0; step < 2 && DEG != kDegFp32; ++step) {   // remainder, then quotient
+        for (int i = n - 2; i >= step; --i) mono[i] += mono[i + 1];
+    }
+    for (int i = 0; i < n; ++i)
+        out->c[i] = static_cast<double>(i == 1 && DEG != kDegFp32 ? -mono[i] : mono[i]);
+    return close_to_shape<DEG, EXACT_U>(ratio, eps, r_s, want, *out);
+}
+
+// What the walk evaluates the pair factor by: the lowest degree whose F is within
+// nine roundings in binary64 (a few ulp, as short_factor_impl) or half an FP32
+// rounding of itself; 0: short_factor_impl. At a softening of r_s / 37, r_cut = 4.5 r_s
+// takes 28 and 12, and short_factor_impl serves binary64 from 6.1 r_s on, where F is
+// 3e-4, or from where softening makes F cross zero (5 r_s at eps = 0.3 r_s); the
+// precision form from 9.5 r_s on at most.
+struct PairForm {
+    int degree = 0;
+    PairPoly poly{};
+};
+constexpr double kWant64 = 2e-15, kWant32 = 6e-8;
+
+PairForm pair_form(const hyowon_treepm_params& P) {
+    PairForm f;
+    PairPoly* const pp = &f.poly;
+    const double ratio = P.cutoff / P.split_scale;
+    if (!(ratio < 10.0)) return f;
+    if (P.precision == HYOWON_FP64) {
+        if (fit_poly<kDegLow, true>(ratio, P.softening, P.split_scale, kWant64, pp)) f.degree = kDegLow;
+        else if (fit_poly<kDegMid, true>(ratio, P.softening, P.split_scale, kWant64, pp)) f.degree = kDegMid;
+        else if (fit_poly<kDegHigh, true>(ratio, P.softening, P.split_scale, kWant64, pp)) f.degree = kDegHigh;
+    } else {
+        if (fit_poly<kDegFp32, false>(ratio, P.softening, P.split_scale, kWant32, pp)) f.degree = kDegFp32;
+        else if (fit_poly<kDegLow, false>(ratio, P.softening, P.split_scale, kWant32, pp)) f.degree = kDegLow;
+        else if (fit_poly<kDegHigh, false>(ratio, P.softening, P.split_scale, kWant32, pp)) f.degree = kDegHigh;
+    }
+    return f;
 }
 
 // Per-particle masses: node mass and centre of mass summed bottom-up, one
@@ -1171,27 +1289,19 @@ void launch_walk_deg(const WalkArgs& A, const PairPoly& pp, int group, cudaStrea
     }
 }
 
-// The lowest polynomial degree that reaches the form's accuracy over the cutoff
-// sphere: below the binary64 rounding of the factor itself, or a tenth of the
-// FP32 one. r_cut = 4.5 r_s takes 20 and 12 (1e-17 and 7e-9); from about
-// r_cut = 7 r_s on (binary64) the closed form stays.
 template <typename R>
-void launch_walk(const WalkArgs& A, int group, cudaStream_t s) {
-    PairPoly pp{};
-    const double ratio = A.W.r_cut / A.W.r_s;
-    const double t_max = ratio * ratio * (1.0 + 1e-9);
-    const long double want = sizeof(R) == 8 ? 1e-16L : 1e-8L;
-    if (t_max < 100.0) {
-        if constexpr (sizeof(R) == 4) {
-            if (fit_poly(kDegLow, t_max, A.W.r_s, &pp) < want)
-                return launch_walk_deg<R, kDegLow>(A, pp, group, s);
-        }
-        if (fit_poly(kDegMid, t_max, A.W.r_s, &pp) < want)
-            return launch_walk_deg<R, kDegMid>(A, pp, group, s);
-        if (fit_poly(kDegHigh, t_max, A.W.r_s, &pp) < want)
-            return launch_walk_deg<R, kDegHigh>(A, pp, group, s);
+void launch_walk(const WalkArgs& A, const PairForm& form, int group, cudaStream_t s) {
+    switch (form.degree) {
+        case kDegFp32:
+            if constexpr (sizeof(R) == 4) launch_walk_deg<R, kDegFp32>(A, form.poly, group, s);
+            break;
+        case kDegLow: launch_walk_deg<R, kDegLow>(A, form.poly, group, s); break;
+        case kDegMid:
+            if constexpr (sizeof(R) == 8) launch_walk_deg<R, kDegMid>(A, form.poly, group, s);
+            break;
+        case kDegHigh: launch_walk_deg<R, kDegHigh>(A, form.poly, group, s); break;
+        default: launch_walk_deg<R, 0>(A, form.poly, group, s);
     }
-    launch_walk_deg<R, 0>(A, pp, group, s);
 }
 
 // Targets a warp takes. A larger group shares the node tests among more targets
@@ -1280,6 +1390,7 @@ int run(const hyowon_treepm_params& P, uint32_t n, const double* x, const double
     uint32_t* level_tmp = mem.get<uint32_t>(scan_tmp_elements(n_counts));
     k_level_counts<<<n_node_tiles, kT, 0, s>>>(n, skey, n_node_tiles, level_hist);
     launch_exclusive_scan(level_hist, level_offs, n_counts, level_tmp, s);
+    const PairForm form = pair_form(P);   // while the device sorts and counts
     uint32_t level_begin[kLevels + 1];   // the last entry: the number of nodes
     TCK(cudaMemcpy2DAsync(level_begin, sizeof(uint32_t), level_offs,
                           sizeof(uint32_t) * n_node_tiles, sizeof(uint32_t), kLevels + 1,
@@ -1342,8 +1453,8 @@ int run(const hyowon_treepm_params& P, uint32_t n, const double* x, const double
                      out_idx, host_targets ? 0 : 1, ax, ay, az, counters, status};
     const int group = walk_group(n, nt);
     cudaEventRecord(ev.e[2], s);
-    if (P.precision == HYOWON_FP64) launch_walk<double>(A, group, s);
-    else launch_walk<float>(A, group, s);
+    if (P.precision == HYOWON_FP64) launch_walk<double>(A, form, group, s);
+    else launch_walk<float>(A, form, group, s);
     TCK(cudaPeekAtLastError());
     cudaEventRecord(ev.e[3], s);
     unsigned long long cnt[2] = {0, 0}, cnt_all[2 * kCounters];

@@ -8,6 +8,8 @@ to 1e-12 relative RMS in binary64 (700 pairs of a few ulp each) and 1e-5 in the
 FP32 form. With theta = 0.5 the same targets give the same accepted set whatever
 the group, so the results agree to summation order (1e-12, and 1e-6 in FP32).
 """
+import math
+
 import numpy as np
 import pytest
 
@@ -45,6 +47,39 @@ def test_pair_factor_over_cutoff_ratios(oracle, precision, ratio):
     ref = oracle.short_range_direct(L, x, y, z, 1.5, t, r_cut / ratio, r_cut, eps)
     got = short_range_forces(L, x, y, z, 1.5, t, r_cut / ratio, r_cut, eps, 1e-6, precision)
     assert rel_rms(got[:3], ref) <= TOL[precision]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("ratio", [2.0, 3.6, 4.5, 5.4, 6.0, 7.0, 7.5, 8.5])
+def test_isolated_pairs_over_the_cutoff_sphere(oracle, precision, ratio):
+    """512 pairs with no other source within reach, their separations spread over the
+    cutoff sphere up to 0.9999 r_cut: each force is one pair factor. Bound, relative to
+    (M_S + |softening term|) / r^3, which the factor equals except where the two cancel
+    (r near 7 r_s): binary64, the factor's own nine roundings, its powers and products
+    (4e-15 in all) and the rounding of r^2 (up to 6 half ulps) times its logarithmic
+    slope, at most 1.5 + q^2 / 4; precision form, 1e-7, the FP32 half ulp and a half."""
+    r_cut, side = 1.0, 8
+    r_s, cell = r_cut / ratio, 3.2 * r_cut
+    eps, L = r_s / 37.0, side * cell
+    rng = np.random.default_rng(int(10 * ratio))
+    n = side ** 3
+    grid = np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij")).reshape(3, n)
+    first = (grid + 0.5) * cell + rng.uniform(-0.05, 0.05, (3, n))
+    way = rng.normal(size=(3, n))
+    r = r_cut * np.concatenate([np.linspace(0.01, 0.9, n // 2), np.linspace(0.9, 0.9999, n - n // 2)])
+    second = first + way / np.linalg.norm(way, axis=0) * r
+    x, y, z = (np.concatenate([a, b]) for a, b in zip(first, second))
+    every = np.arange(2 * n, dtype=np.uint32)
+    args = (r_s, r_cut, eps)
+    ref = np.stack(oracle.short_range_direct(L, x, y, z, 1.0, every, *args))
+    got = np.stack(short_range_forces(L, x, y, z, 1.0, every, *args, 1e-6, precision)[:3])
+    q = np.tile(r, 2) / r_s
+    ms = np.array([math.erfc(0.5 * v) for v in q]) + q / math.sqrt(math.pi) * np.exp(-0.25 * q * q)
+    soft = np.expm1(-1.5 * np.log1p((eps / r_s / q) ** 2))
+    scale = np.linalg.norm(ref, axis=0) * (ms - soft) / np.abs(ms + soft)
+    err = np.linalg.norm(got - ref, axis=0) / scale
+    bound = (1.5 + 0.25 * q * q) * 6.7e-16 + 4e-15 if precision == "fp64" else 1e-7
+    assert np.all(err <= bound), (float(np.max(err)), float(np.max(err / bound)))
 
 
 @pytest.mark.parametrize("n,nt", [(2, 1), (2, 2), (3, 3), (5, 5), (17, 17), (33, 31), (4097, 4097),
