@@ -1396,11 +1396,17 @@ int run(const hyowon_treepm_params& P, uint32_t n, const double* x, const double
                           sizeof(uint32_t) * n_node_tiles, sizeof(uint32_t), kLevels + 1,
                           cudaMemcpyDeviceToHost, s));
     TCK(cudaStreamSynchronize(s));
-    const uint32_t node_base = level_begin[kLevels];
-    if (node_base > 6ull * n + 64) throw Fail{HYOWON_ERUNTIME, "octree node capacity exceeded"};
+    // A level has at most n nodes, so the differences are its counts even where the
+    // 32-bit running total wrapped; only a total that needs more bits is refused.
+    uint64_t total = 0;
     int depth = 0;
-    for (int l = 1; l < kLevels; ++l)
-        if (level_begin[l + 1] > level_begin[l]) depth = l;
+    for (int l = 0; l < kLevels; ++l) {
+        const uint32_t here = level_begin[l + 1] - level_begin[l];
+        total += here;
+        if (here) depth = l;
+    }
+    if (total > 0xFFFFFFF0ull) throw Fail{HYOWON_ERUNTIME, "octree of more than 2^32-16 nodes"};
+    const uint32_t node_base = static_cast<uint32_t>(total);
     Node* nodes = mem.get<Node>(node_base);
     k_emit_nodes<<<n_node_tiles, kT, 0, s>>>(n, skey, n_node_tiles, level_offs, P.box_size, sx, sy,
                                              sz, pq[0], pq[1], pq[2], P.particle_mass, nodes);

@@ -176,3 +176,20 @@ def test_tree_of_tile_edges_and_coincident_sources(oracle, n, copies):
     ref = oracle.short_range_direct(L, x, y, z, 1.0, every, r_cut / 4.5, r_cut, eps)
     scale = max(float(np.max(np.abs(r))) for r in ref)
     assert max(float(np.max(np.abs(g - r))) for g, r in zip(got[:3], ref)) <= 1e-12 * max(scale, 1e-300)
+
+
+def test_tree_of_tight_pairs_alone(oracle):
+    """1000 pairs 1e-6 L apart: each hangs on a chain of single-child nodes, nine nodes
+    a source in all. Node count from the definition, forces from direct summation."""
+    L, r_cut, eps, n = 20.0, 6.0, 0.02, 1000
+    rng = np.random.default_rng(8)
+    first = rng.uniform(0.01 * L, 0.99 * L, (3, n))
+    way = rng.normal(size=(3, n))
+    second = first + 1e-6 * L * way / np.linalg.norm(way, axis=0)
+    x, y, z = (np.concatenate([a, b]) for a, b in zip(first, second))
+    every = np.arange(2 * n, dtype=np.uint32)
+    got = short_range_forces(L, x, y, z, 1.0, every, r_cut / 4.5, r_cut, eps, 1e-6)
+    assert (int(got[3]["nodes"]), int(got[3]["depth"])) == tree_size(L, x, y, z)
+    assert got[3]["nodes"] > 6 * 2 * n + 64
+    ref = oracle.short_range_direct(L, x, y, z, 1.0, every, r_cut / 4.5, r_cut, eps)
+    assert rel_rms(got[:3], ref) <= TOL["fp64"]
