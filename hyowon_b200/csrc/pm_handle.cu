@@ -1586,6 +1586,12 @@ int hyowon_pm_debug_set_wait_limit(hyowon_pm_t h, unsigned polls) {
     return HYOWON_OK;
 }
 
+int hyowon_pm_debug_tree_allocations(hyowon_pm_t h, uint64_t* count) {
+    if (!h || !count) return HYOWON_EINVAL;
+    *count = tree::workspace_allocations(h->tree_ws);
+    return HYOWON_OK;
+}
+
 int hyowon_pm_debug_offset_mass_target(hyowon_pm_t h, double delta) {
     if (!h || !std::isfinite(delta)) return HYOWON_EINVAL;
     h->mass_target_offset = delta;

@@ -1192,11 +1192,22 @@ struct Fail {
 // carved from (256-byte aligned), so that repeated solves allocate nothing.
 // A call that needs more than it holds takes the rest from cudaMalloc and
 // records the total, and the next call regrows the block to that size.
+//
+// The node arrays' size is known only within the call, and a clustering run's tree
+// grows from step to step (1.39 n nodes near a lattice, 1.46 n clustered): they are
+// carved for `nodes` nodes, at least 2 n and a fourth more than any tree that went
+// beyond that had. Sized exactly, a larger tree cost its solve 36 ms and the next 7
+// (4.1M sources, whose build takes 2.0). Where memory is too short, exactly.
 struct Workspace {
     void* base = nullptr;
     size_t cap = 0;
     size_t want = 0;
+    uint32_t nodes = 0;
+    bool exact = false;
+    uint64_t allocations = 0;   // cudaMalloc calls made for it
 };
+
+uint64_t workspace_allocations(const Workspace* ws) { return ws ? ws->allocations : 0; }
 
 Workspace* create_workspace() { return new (std::nothrow) Workspace(); }
 
@@ -1218,9 +1229,46 @@ struct Mem {
             if (ws->base) cudaFree(ws->base);
             ws->base = nullptr;
             ws->cap = 0;
-            TCK(cudaMalloc(&ws->base, ws->want));
+            if (!allocate(&ws->base, ws->want)) {
+                // buffer by buffer instead, and without room for a larger tree
+                ws->want = 0;
+                ws->exact = true;
+                return;
+            }
             ws->cap = ws->want;
         }
+    }
+    // Nodes that the node arrays of a tree of n_nodes on n sources are carved for.
+    uint32_t node_room(uint32_t n, uint32_t n_nodes) {
+        if (!ws || ws->exact) return n_nodes;
+        if (n_nodes > ws->nodes || n > ws->nodes / 2) {
+            const uint64_t room = std::max<uint64_t>(2ull * n, n_nodes + n_nodes / 4ull);
+            ws->nodes = static_cast<uint32_t>(std::min<uint64_t>(room, 0xFFFFFFF0ull));
+        }
+        return std::max(ws->nodes, n_nodes);
+    }
+    bool allocate(void** q, size_t bytes) {
+        if (ws) ++ws->allocations;
+        const cudaError_t e = cudaMalloc(q, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            return false;
+        }
+        TCK(e);
+        return true;
+    }
+    // `count` elements, or at least `least` where memory is short.
+    template <typename T>
+    T* get_room(size_t count, size_t least) {
+        const size_t at = off;
+        try {
+            return get<T>(count);
+        } catch (const Fail& f) {
+            if (f.code != HYOWON_ENOMEM || count <= least) throw;
+        }
+        ws->exact = true;
+        off = at;
+        return get<T>(least);
     }
     template <typename T>
     T* get(size_t count) {
@@ -1231,7 +1279,7 @@ struct Mem {
             if (off <= ws->cap) return reinterpret_cast<T*>(static_cast<char*>(ws->base) + at);
         }
         void* q = nullptr;
-        TCK(cudaMalloc(&q, bytes));
+        if (!allocate(&q, bytes)) throw Fail{HYOWON_ENOMEM, "octree work arrays could not be allocated"};
         p.push_back(q);
         return static_cast<T*>(q);
     }
@@ -1407,7 +1455,8 @@ int run(const hyowon_treepm_params& P, uint32_t n, const double* x, const double
     }
     if (total > 0xFFFFFFF0ull) throw Fail{HYOWON_ERUNTIME, "octree of more than 2^32-16 nodes"};
     const uint32_t node_base = static_cast<uint32_t>(total);
-    Node* nodes = mem.get<Node>(node_base);
+    const uint32_t room = mem.node_room(n, node_base);
+    Node* nodes = mem.get_room<Node>(room, node_base);
     k_emit_nodes<<<n_node_tiles, kT, 0, s>>>(n, skey, n_node_tiles, level_offs, P.box_size, sx, sy,
                                              sz, pq[0], pq[1], pq[2], P.particle_mass, nodes);
     if (sm) {
@@ -1416,9 +1465,9 @@ int run(const hyowon_treepm_params& P, uint32_t n, const double* x, const double
             k_moments<<<nb(e - b), kT, 0, s>>>(b, e, sx, sy, sz, sm, nodes);
         }
     }
-    uint4* ga = mem.get<uint4>(node_base);
-    uint4* gm = mem.get<uint4>(node_base);
-    uint4* gc = mem.get<uint4>(node_base);
+    uint4* ga = mem.get_room<uint4>(room, node_base);
+    uint4* gm = mem.get_room<uint4>(room, node_base);
+    uint4* gc = mem.get_room<uint4>(room, node_base);
     k_walk_nodes<<<nb(node_base), kT, 0, s>>>(node_base, P.theta, P.box_size, nodes, ga, gm, gc);
     cudaEventRecord(ev.e[1], s);
     const uint32_t* dslots = nullptr;

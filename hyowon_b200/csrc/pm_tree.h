@@ -16,6 +16,7 @@ namespace hyowon::tree {
 struct Workspace;
 Workspace* create_workspace();
 void destroy_workspace(Workspace* ws);
+uint64_t workspace_allocations(const Workspace* ws);   // cudaMalloc calls made for it
 
 // Octree of the n device sources (x, y, z in [0, L) after wrapping; masses or,
 // when null, P.particle_mass) and the short-range walk of every source as a

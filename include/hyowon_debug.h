@@ -1,5 +1,5 @@
 /*
- * hyowon_debug.h -- failure injection for tests of the error paths.
+ * hyowon_debug.h -- failure injection and counters for tests.
  *
  * No counterpart in the reference. These calls make the handle's own bounded
  * checks fail from the host, so that tests can see a failure reported as a
@@ -30,6 +30,10 @@ int hyowon_pm_debug_set_wait_limit(hyowon_pm_t h, unsigned polls);
  * the precision form its exact fixed-point mesh sum with the expected sum
  * plus delta units. 0 restores the exact target. */
 int hyowon_pm_debug_offset_mass_target(hyowon_pm_t h, double delta);
+
+/* cudaMalloc calls made so far for the octree's work arrays of this handle (a
+ * clustering run makes none from its third solve on). */
+int hyowon_pm_debug_tree_allocations(hyowon_pm_t h, uint64_t* count);
 
 #ifdef __cplusplus
 }

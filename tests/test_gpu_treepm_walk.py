@@ -8,12 +8,14 @@ to 1e-12 relative RMS in binary64 (700 pairs of a few ulp each) and 1e-5 in the
 FP32 form. With theta = 0.5 the same targets give the same accepted set whatever
 the group, so the results agree to summation order (1e-12, and 1e-6 in FP32).
 """
+import ctypes
 import math
 
 import numpy as np
 import pytest
 
 import hyowon_b200 as hb
+from hyowon_b200 import _native as nat
 from hyowon_b200.treepm import short_range_forces
 
 pytestmark = pytest.mark.gpu
@@ -193,3 +195,37 @@ def test_tree_of_tight_pairs_alone(oracle):
     assert got[3]["nodes"] > 6 * 2 * n + 64
     ref = oracle.short_range_direct(L, x, y, z, 1.0, every, r_cut / 4.5, r_cut, eps)
     assert rel_rms(got[:3], ref) <= TOL["fp64"]
+
+
+def test_growing_tree_allocates_once():
+    """One handle whose tree grows from solve to solve, as in a clustering run: after two
+    solves the work arrays hold it (up to two nodes a source; once more for a tree beyond
+    that), and the forces are those of a fresh handle, bit for bit."""
+    L, side, r_s = 20.0, 27, 0.25
+    n = side ** 3
+    rng = np.random.default_rng(12)
+    grid = (np.stack(np.meshgrid(*[np.arange(side)] * 3, indexing="ij")).reshape(3, n) + 0.5) * L / side
+    grid += rng.uniform(-0.2, 0.2, (3, n)) * L / side
+    clump = rng.uniform(0, L, (3, 40))[:, rng.integers(0, 40, n)] + rng.normal(0, 0.15, (3, n))
+    pair = rng.uniform(0, L, (3, n))
+    pair[:, 1::2] = pair[:, :n - 1:2] + 3e-6 * L * rng.uniform(-1, 1, (3, n // 2))
+    states = [np.where(np.arange(n) < f * n, clump, grid) for f in (0.0, 0.2, 0.4, 0.6, 0.9)]
+    states += [pair, pair, grid, pair]
+    geometry, method = hb.MeshGeometry(L, 32), hb.PMForceMethod.treepm_long_range(r_s)
+    made, nodes = [], []
+    count = ctypes.c_uint64()
+    with hb.PMSolver(geometry, method) as s:
+        for p in states:
+            x, y, z = np.mod(p, L)
+            s.upload(x, y, z, uniform_mass=1.0)
+            got = s.treepm_short_forces(0.5, 0.03, 4.5 * r_s)
+            assert nat.lib().hyowon_pm_debug_tree_allocations(s.handle, ctypes.byref(count)) == 0
+            made.append(count.value)
+            nodes.append(got[3]["nodes"])
+            with hb.PMSolver(geometry, method) as fresh:
+                fresh.upload(x, y, z, uniform_mass=1.0)
+                want = fresh.treepm_short_forces(0.5, 0.03, 4.5 * r_s)
+            assert all(np.array_equal(g, w) for g, w in zip(got[:3], want[:3]))
+    assert all(a < b for a, b in zip(nodes[:5], nodes[1:5])) and nodes[4] < 2 * n < nodes[5]
+    assert made[1] == made[4], made          # grown trees of up to 2 n nodes
+    assert made[6] == made[8], made          # beyond: one call past the block, one regrow
