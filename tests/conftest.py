@@ -30,6 +30,14 @@ def oracle():
     return Oracle()
 
 
+def reference_or_skip():
+    """The reference's own build, or a skip where its sources are not here to build it."""
+    from oracle.bindings import REF_SO, Reference, build_reference
+    if not os.path.exists(REF_SO) and not build_reference():
+        pytest.skip("the reference is not built and its source tree is absent")
+    return Reference()
+
+
 @pytest.fixture(scope="session")
 def small_pm():
     return load_golden("small_pm.npz")

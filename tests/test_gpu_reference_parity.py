@@ -30,6 +30,7 @@ import numpy as np
 import pytest
 
 import hyowon_b200 as hb
+from conftest import reference_or_skip
 
 pytestmark = pytest.mark.gpu
 
@@ -49,8 +50,7 @@ def pos_rms_cells(a, b, L, N):
 
 @pytest.fixture(scope="module")
 def reference():
-    from oracle.bindings import Reference
-    return Reference()
+    return reference_or_skip()
 
 
 @pytest.fixture(scope="module")

@@ -24,6 +24,7 @@ import numpy as np
 import pytest
 
 import hyowon_b200 as hb
+from conftest import reference_or_skip
 from hyowon_b200 import treepm
 
 pytestmark = pytest.mark.gpu
@@ -48,8 +49,7 @@ def pos_rms_cells(a, b):
 @pytest.fixture(scope="module")
 def setup():
     from oracle import workload
-    from oracle.bindings import Reference
-    ref = Reference()
+    ref = reference_or_skip()
     st = workload.reference_ics(ref, "c1", n_side=NS, box=L)
     ics = {k: np.array(st[k]) for k in COMPS}
     m_lat = workload.particle_mass(L, NS)
