@@ -289,7 +289,11 @@ def run_reference(args, world, rank):
     from oracle.bindings import Reference
     cfg_name = args.config
     c = workload.CONFIGS[cfg_name]
-    ref = Reference()
+    try:
+        ref = Reference()
+    except OSError as e:   # not built, or its libraries are not here
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+        return
     a0, dl = workload.schedule(cfg_name)
     n_side = c["n_side"]
     st = workload.reference_ics(ref, cfg_name)

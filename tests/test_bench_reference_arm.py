@@ -28,3 +28,13 @@ def test_reference_arm_loads_only_the_reference_build():
     assert line["value"] > 0 and line["steps"] == 2
     assert line["cpu_baseline"]["kind"] == "reference"
     assert line["e2e"]["h2d_bytes_per_step"] == 0
+
+
+@pytest.mark.skipif(os.path.exists(os.path.join(ROOT, "oracle", "_ref", "libhyowon_ref.so")),
+                    reason="the reference build is present")
+def test_reference_arm_says_so_when_it_cannot_run():
+    out = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference",
+                          "--config", "c1", "--steps", "2"], cwd=ROOT, capture_output=True, text=True,
+                         timeout=300, check=True).stdout
+    line = json.loads([ln for ln in out.splitlines() if ln.startswith("{")][-1])
+    assert line["impl"] == "reference" and "not built" in line["unavailable"]
