@@ -605,6 +605,10 @@ public:
         return base_ ? reinterpret_cast<T*>(base_ + at) : nullptr;
     }
     size_t capacity() const { return cap_; }
+    // Where the next array goes; reach() makes the layout at least that long.
+    size_t offset() const { return off_; }
+    void* at(size_t offset) const { return base_ ? base_ + offset : nullptr; }
+    void reach(size_t offset) { off_ = off_ > offset ? off_ : (offset + 255) & ~static_cast<size_t>(255); }
     void release() {
         cudaFree(block_);
         block_ = nullptr;
@@ -739,8 +743,8 @@ public:
     // Gives the work arrays of a run back; the next run takes them again.
     void trim() {
         cudaStreamSynchronize(s_);
-        arena_.release();
         lpt_.release();
+        arena_.release();
     }
 
     ~Engine() {
@@ -833,15 +837,24 @@ public:
         R *u[3] = {}, *psi = nullptr, *field = nullptr, *kept_block = nullptr;
         std::vector<double*> cx(3 * n_ckpt);
         std::vector<R*> cp(3 * n_ckpt);
+        const char* err = nullptr;
+        if (const int rc = lpt_.plan(static_cast<int>(cfg_.n_side), &err))
+            throw Fail{rc, err ? err : "LPT failed"};
+        void* lpt_at = nullptr;
         bool keep = false;
         auto layout = [&] {
             d_noise = arena_.template take<double>(n_);
             tab = arena_.template take<double>(3 * cfg_.n_nodes);
             for (int a = 0; a < 3; ++a) pd[a] = arena_.template take<double>(n_);
+            // The 1LPT map runs before the first checkpoint is written and its adjoint
+            // after the last is read: their arrays take the checkpoints' place.
+            const size_t first = arena_.offset();
+            lpt_at = arena_.at(first);
             for (uint64_t c = 0; c < 3 * n_ckpt; ++c) {
                 cx[c] = arena_.template take<double>(n_);
                 cp[c] = arena_.template take<R>(n_);
             }
+            arena_.reach(first + lpt_.bytes);
             if (want_grad) {
                 for (int a = 0; a < 3; ++a) {
                     lx[a] = arena_.template take<double>(n_);
@@ -861,11 +874,6 @@ public:
         // device memory allows: the reverse pass then re-derives each state's
         // force by one gather instead of a deposit and a Green's-function
         // solve. Particle states stay checkpointed every k steps either way.
-        {
-            const char* lerr = nullptr;
-            const int wrc = lpt_.require(static_cast<int>(cfg_.n_side), s_, &lerr);
-            if (wrc) throw Fail{wrc, lerr ? lerr : "LPT failed"};
-        }
         if (want_grad) {
             const size_t rest = arena_.count(layout);
             size_t free_b = 0, total_b = 0;
@@ -875,18 +883,18 @@ public:
                 && need + (size_t(1) << 30) < (free_b + arena_.capacity() - rest) / 2;
         }
         arena_.plan(layout);
+        lpt_.place(lpt_at);
         // A block of more than 1/32 of the device's memory is given back.
         struct GiveBack {
-            Arena& a;
-            cudaStream_t s;
+            Engine& e;
             ~GiveBack() {
                 size_t free_b = 0, total_b = 0;
-                if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || a.capacity() > total_b / 32) {
-                    cudaStreamSynchronize(s);
-                    a.release();
-                }
+                e.lpt_.place(nullptr);
+                if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess
+                    || e.arena_.capacity() > total_b / 32)
+                    e.trim();
             }
-        } give_back{arena_, s_};
+        } give_back{*this};
         std::vector<R*> kept;
         if (keep)
             for (uint64_t j = 0; j <= S; ++j) kept.push_back(kept_block + j * phi_stride);
@@ -912,7 +920,6 @@ public:
         ACK(cudaMemcpyAsync(tab + 2 * cfg_.n_nodes, cfg_.ln_p_y2, sizeof(double) * cfg_.n_nodes, cudaMemcpyHostToDevice, s_));
         if (target)
             ACK(cudaMemcpyAsync(d_target, target, sizeof(double) * cells_, cudaMemcpyHostToDevice, s_));
-        const char* err = nullptr;
         const int lrc = lpt_ics_device(lpt_, static_cast<int>(cfg_.n_side), cfg_.box_size, d_noise, tab,
                                        tab + cfg_.n_nodes, tab + 2 * cfg_.n_nodes,
                                        static_cast<int>(cfg_.n_nodes), cfg_.momentum_factor, x_, pd,

@@ -160,47 +160,57 @@ __global__ void k_scale(uint64_t n, const double* __restrict__ in, double s, dou
 
 static_assert(sizeof(cufftHandle) == sizeof(int), "LptWork keeps plan handles as int");
 
-int LptWork::require(int n_side, cudaStream_t s, const char** err) {
+int LptWork::plan(int n_side, const char** err) {
     *err = nullptr;
-    if (N != n_side || !plans) {
+    if (N == n_side && plans) return 0;
+    release();
+    const size_t cells = static_cast<size_t>(n_side) * n_side * n_side;
+    const size_t half = static_cast<size_t>(n_side) * n_side * (n_side / 2 + 1);
+    size_t w1 = 0, w2 = 0;
+    if (cufftCreate(&r2c) != CUFFT_SUCCESS) {
+        *err = "cufftCreate failed";
+        return 6;
+    }
+    if (cufftCreate(&c2r) != CUFFT_SUCCESS) {
+        cufftDestroy(r2c);
+        *err = "cufftCreate failed";
+        return 6;
+    }
+    plans = true;
+    cufftSetAutoAllocation(r2c, 0);
+    cufftSetAutoAllocation(c2r, 0);
+    if (cufftMakePlan3d(r2c, n_side, n_side, n_side, CUFFT_D2Z, &w1) != CUFFT_SUCCESS
+        || cufftMakePlan3d(c2r, n_side, n_side, n_side, CUFFT_Z2D, &w2) != CUFFT_SUCCESS) {
+        *err = "cuFFT plan for the IC mesh failed";
         release();
-        const size_t cells = static_cast<size_t>(n_side) * n_side * n_side;
-        const size_t half = static_cast<size_t>(n_side) * n_side * (n_side / 2 + 1);
-        size_t w1 = 0, w2 = 0;
-        if (cufftCreate(&r2c) != CUFFT_SUCCESS) {
-            *err = "cufftCreate failed";
-            release();
-            return 6;
-        }
-        if (cufftCreate(&c2r) != CUFFT_SUCCESS) {
-            cufftDestroy(r2c);
-            *err = "cufftCreate failed";
-            release();
-            return 6;
-        }
-        plans = true;
-        cufftSetAutoAllocation(r2c, 0);
-        cufftSetAutoAllocation(c2r, 0);
-        if (cufftMakePlan3d(r2c, n_side, n_side, n_side, CUFFT_D2Z, &w1) != CUFFT_SUCCESS
-            || cufftMakePlan3d(c2r, n_side, n_side, n_side, CUFFT_Z2D, &w2) != CUFFT_SUCCESS) {
-            *err = "cuFFT plan for the IC mesh failed";
-            release();
-            return 6;
-        }
-        const size_t spectrum = (sizeof(double2) * half + 255) & ~static_cast<size_t>(255);
-        const size_t mesh = (sizeof(double) * cells + 255) & ~static_cast<size_t>(255);
-        if (cudaMalloc(&block, 2 * spectrum + mesh + (w1 > w2 ? w1 : w2)) != cudaSuccess) {
+        return 6;
+    }
+    N = n_side;
+    spectrum = (sizeof(double2) * half + 255) & ~static_cast<size_t>(255);
+    mesh = (sizeof(double) * cells + 255) & ~static_cast<size_t>(255);
+    bytes = 2 * spectrum + mesh + (w1 > w2 ? w1 : w2);
+    return 0;
+}
+
+void LptWork::place(void* at) {
+    char* const p = static_cast<char*>(at);
+    delta = reinterpret_cast<double2*>(p);
+    work = p ? reinterpret_cast<double2*>(p + spectrum) : nullptr;
+    real = p ? reinterpret_cast<double*>(p + 2 * spectrum) : nullptr;
+    if (!p) return;
+    cufftSetWorkArea(r2c, p + 2 * spectrum + mesh);
+    cufftSetWorkArea(c2r, p + 2 * spectrum + mesh);
+}
+
+int LptWork::require(int n_side, cudaStream_t s, const char** err) {
+    if (const int rc = plan(n_side, err)) return rc;
+    if (!delta) {
+        if (cudaMalloc(&block, bytes) != cudaSuccess) {
             *err = "LPT work arrays could not be allocated";
             release();
             return 7;
         }
-        char* at = static_cast<char*>(block);
-        delta = reinterpret_cast<double2*>(at);
-        work = reinterpret_cast<double2*>(at + spectrum);
-        real = reinterpret_cast<double*>(at + 2 * spectrum);
-        cufftSetWorkArea(r2c, at + 2 * spectrum + mesh);
-        cufftSetWorkArea(c2r, at + 2 * spectrum + mesh);
-        N = n_side;
+        place(block);
     }
     cufftSetStream(r2c, s);
     cufftSetStream(c2r, s);
@@ -218,6 +228,7 @@ void LptWork::release() {
     delta = work = nullptr;
     real = nullptr;
     N = 0;
+    bytes = 0;
 }
 
 int lpt_adjoint_device(LptWork& w, int N, double L, double* const d_g[3], const double* d_xs,

@@ -6,16 +6,24 @@
 namespace hyowon {
 
 // Transform plans and work arrays of the 1LPT map and its adjoint on one lattice
-// side; made on first use, freed with the object (or by release()).
+// side. The arrays are the caller's (place()), or a block of their own that is made
+// on first use and freed with the object or by release().
 struct LptWork {
     int N = 0;
-    void* block = nullptr;      // one allocation: the arrays below and cuFFT's own
+    size_t bytes = 0;           // what the arrays below and cuFFT's own take
+    size_t spectrum = 0, mesh = 0;   // of which a half spectrum and the mesh
     double2* delta = nullptr;   // half spectra
     double2* work = nullptr;
     double* real = nullptr;
     int r2c = 0, c2r = 0;       // cufftHandle
     bool plans = false;
-    // 0, 6 (CUDA / cuFFT) or 7 (allocation); *err names the failure.
+    void* block = nullptr;      // the block of its own, if any
+    // Plans for n_side, and `bytes`. 0 or 6 (cuFFT); *err names the failure.
+    int plan(int n_side, const char** err);
+    // Puts the arrays into `bytes` bytes of the caller's, 256-byte aligned, used by the
+    // calls below until they return; null takes them out again.
+    void place(void* at);
+    // plan(), with a block of its own unless the arrays are placed. 0, 6 or 7 (allocation).
     int require(int n_side, cudaStream_t s, const char** err);
     void release();
     LptWork() = default;

@@ -62,3 +62,21 @@ def test_vjp_before_and_after_other_work_of_the_handle(precision):
         check(s, box, n, N, 3, 2, precision, 2)
         s.kdk_step(f[0][1], f[1][1], f[2][1])
         check(s, box, n, N, 3, 2, precision, 3)
+
+
+def test_large_lattice_leaves_the_engine_alone():
+    """A 512^3 lattice: a run's work arrays, the 1LPT ones (5 GB) among them, exceed a 32nd
+    of the device's memory and are given back after the call; positions, momenta and
+    accelerations (48 bytes a particle in FP32) and the small mesh stay."""
+    import torch
+    box, n, N = 60.0, 512, 32
+    rng = np.random.default_rng(3)
+    noise = np.tile(rng.standard_normal(n * n), n)
+    target = np.zeros(N ** 3)
+    with hb.PMSolver(hb.MeshGeometry(box, N), hb.PMForceMethod.pure_pm(False), "fp32") as s:
+        free, _ = torch.cuda.mem_get_info()
+        d = adjoint.DifferentiablePM(box, n, N, 0.05, 1, "fp32", 1, solver=s)
+        first = d.loss(noise, target)
+        held = free - torch.cuda.mem_get_info()[0]
+        assert abs(held - 48 * n ** 3) <= 256 << 20, held
+        assert abs(d.loss(noise, target) - first) <= TOL["fp32"] * abs(first)
