@@ -519,18 +519,38 @@ k_columns(const __grid_constant__ CUtensorMap map, cx_t<T>* __restrict__ H,
     }
 }
 
+// A number of the current context that no other context of the process has or had
+// (a kernel's shared-memory allowance belongs to the context, and device reset or a
+// second context starts from the default); 0 where the driver does not say.
+unsigned long long context_id() {
+    using CtxGetId = CUresult (*)(CUcontext, unsigned long long*);
+    static const CtxGetId fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPoint("cuCtxGetId", &f, cudaEnableDefault, &q) != cudaSuccess
+            || q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            return static_cast<CtxGetId>(nullptr);
+        }
+        return reinterpret_cast<CtxGetId>(f);
+    }();
+    unsigned long long id = 0;
+    return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
 // Resident blocks of a kernel on the whole device, its dynamic shared memory
-// allowed; worked out once per kernel and device (five runtime calls, some 5 us,
-// that every launch made). 0 on failure.
+// allowed; worked out once per kernel, device and context (five runtime calls, some
+// 5 us, that every launch made). 0 on failure.
 template <auto KERNEL>
 unsigned resident_blocks(int threads, size_t smem) {
-    static std::atomic<unsigned> known[64];
+    static std::atomic<unsigned long long> known[64];   // context id << 24 | blocks
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    const bool slot = dev >= 0 && dev < 64;
+    const unsigned long long context = context_id();
+    const bool slot = dev >= 0 && dev < 64 && context != 0 && context < 1ull << 40;
     if (slot) {
-        const unsigned k = known[dev].load(std::memory_order_acquire);
-        if (k) return k;
+        const unsigned long long k = known[dev].load(std::memory_order_acquire);
+        if (k >> 24 == context) return static_cast<unsigned>(k & 0xffffffu);
     }
     int sms = 0, per_sm = 0;
     if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -540,7 +560,7 @@ unsigned resident_blocks(int threads, size_t smem) {
         || per_sm < 1)
         return 0;
     const unsigned full = static_cast<unsigned>(sms) * static_cast<unsigned>(per_sm);
-    if (slot) known[dev].store(full, std::memory_order_release);
+    if (slot && full < 1u << 24) known[dev].store(context << 24 | full, std::memory_order_release);
     return full;
 }
 
