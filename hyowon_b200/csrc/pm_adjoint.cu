@@ -824,6 +824,7 @@ public:
              double* delta_out, double* timings) {
         const uint64_t S = cfg_.n_steps;
         const uint64_t k = cfg_.ckpt_every > 0 ? cfg_.ckpt_every : 1;
+        solves_ = vjps_ = 0;
         Events ev;
         const cudaEvent_t e0 = ev.e[0], e1 = ev.e[1], e2 = ev.e[2];
         ACK(cudaMemsetAsync(status_, 0, sizeof(unsigned int), s_));

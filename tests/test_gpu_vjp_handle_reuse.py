@@ -80,3 +80,19 @@ def test_large_lattice_leaves_the_engine_alone():
         held = free - torch.cuda.mem_get_info()[0]
         assert abs(held - 48 * n ** 3) <= 256 << 20, held
         assert abs(d.loss(noise, target) - first) <= TOL["fp32"] * abs(first)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_counts_are_those_of_the_call(precision):
+    """Force solves and force VJPs reported by repeated calls on a handle."""
+    box, n, N = 60.0, 16, 32
+    noise, target = inputs(n, N, 1)
+    args = (box, n, N, 0.05, 4, precision, 2)
+    alone = adjoint.DifferentiablePM(*args)
+    alone.loss_and_grad(noise, target)
+    want = {k: alone.last_timings[k] for k in ("force_solves", "force_vjps")}
+    with hb.PMSolver(hb.MeshGeometry(box, N), hb.PMForceMethod.pure_pm(False), precision) as s:
+        d = adjoint.DifferentiablePM(*args, solver=s)
+        for _ in range(3):
+            d.loss_and_grad(noise, target)
+            assert {k: d.last_timings[k] for k in want} == want
