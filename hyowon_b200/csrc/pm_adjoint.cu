@@ -29,6 +29,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <new>
 #include <string>
 #include <vector>
@@ -1099,8 +1100,8 @@ int run_cached(Cache** cache, const VjpConfig& cfg, cudaStream_t s, const double
     } catch (const Fail& f) {
         if (err) *err = f.msg;
         return f.code;
-    } catch (const std::bad_alloc&) {
-        if (err) *err = "out of host memory";
+    } catch (const std::exception& e) {   // bad_alloc, length_error
+        if (err) *err = std::string("out of host memory: ") + e.what();
         return HYOWON_ENOMEM;
     }
     return HYOWON_OK;
@@ -1149,6 +1150,9 @@ int hyowon_vjp_1lpt_pm(const hyowon_vjp_config* cfg, const double* noise,
     } catch (const Fail& f) {
         g_adj_err = f.msg;
         rc = f.code;
+    } catch (const std::exception& e) {   // bad_alloc, length_error
+        g_adj_err = std::string("out of host memory: ") + e.what();
+        rc = HYOWON_ENOMEM;
     }
     cudaStreamDestroy(s);
     return rc;

@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <exception>
 #include <limits>
 #include <new>
 #include <string>
@@ -1571,6 +1572,9 @@ int device_short_forces(const hyowon_treepm_params& P, uint32_t n, const double*
     } catch (const Fail& f) {
         if (err) *err = f.msg;
         return f.code;
+    } catch (const std::exception& e) {   // bad_alloc, length_error
+        if (err) *err = std::string("out of host memory: ") + e.what();
+        return HYOWON_ENOMEM;
     }
 }
 
@@ -1605,6 +1609,9 @@ int hyowon_treepm_short_forces(const hyowon_treepm_params* params, uint64_t n, c
     } catch (const Fail& f) {
         g_err = f.msg;
         return f.code;
+    } catch (const std::exception& e) {   // bad_alloc, length_error
+        g_err = std::string("out of host memory: ") + e.what();
+        return HYOWON_ENOMEM;
     }
 }
 

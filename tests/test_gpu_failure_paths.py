@@ -10,12 +10,15 @@
   solve fail with the reference's runtime error (src/math/cic_mass_conservation.cpp:41-59);
   with the target restored the handle solves again.
 Both forms, on a power-of-two mesh (the five-pass solve) of 64^3 cells.
+* A gradient of more steps than host memory holds checkpoints for is an
+  out-of-memory error of the call, stateless or on a handle; the handle works on.
 """
 import numpy as np
 import pytest
 
 import hyowon_b200 as hb
 from hyowon_b200 import _native as nat
+from hyowon_b200 import adjoint
 
 pytestmark = pytest.mark.gpu
 
@@ -63,3 +66,25 @@ def test_mass_conservation_violation_is_reported_and_recovered(form):
         got = s.download()
     for k in ("ax", "ay", "az"):
         assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("form", ["fp64", "fp32"])
+def test_gradient_of_too_many_steps_is_an_error(form):
+    box, n, N = 60.0, 16, 32
+    rng = np.random.default_rng(2)
+    noise, target = rng.standard_normal(n ** 3), 0.3 * rng.standard_normal(N ** 3)
+
+    class Endless(adjoint.DifferentiablePM):
+        def _cfg(self):   # refused before the schedule is read
+            c = super()._cfg()
+            c.n_steps = 1 << 60
+            return c
+
+    args = (box, n, N, 0.05, 3, form, 1)
+    with pytest.raises(MemoryError):
+        Endless(*args).loss_and_grad(noise, target)
+    with hb.PMSolver(hb.MeshGeometry(box, N), hb.PMForceMethod.pure_pm(False), form) as s:
+        with pytest.raises(MemoryError):
+            Endless(*args, solver=s).loss_and_grad(noise, target)
+        got = adjoint.DifferentiablePM(*args, solver=s).loss_and_grad(noise, target)
+    assert np.isfinite(got[0]) and np.all(np.isfinite(got[1]))
