@@ -12,13 +12,15 @@
 Both forms, on a power-of-two mesh (the five-pass solve) of 64^3 cells.
 * A gradient of more steps than host memory holds checkpoints for is an
   out-of-memory error of the call, stateless or on a handle; the handle works on.
+* A solve whose particles cannot be keyed (1LPT of non-finite noise) is refused
+  after the sort was already enqueued: the particle arrays stay as they were.
 """
 import numpy as np
 import pytest
 
 import hyowon_b200 as hb
 from hyowon_b200 import _native as nat
-from hyowon_b200 import adjoint
+from hyowon_b200 import adjoint, ic
 
 pytestmark = pytest.mark.gpu
 
@@ -88,3 +90,29 @@ def test_gradient_of_too_many_steps_is_an_error(form):
             Endless(*args, solver=s).loss_and_grad(noise, target)
         got = adjoint.DifferentiablePM(*args, solver=s).loss_and_grad(noise, target)
     assert np.isfinite(got[0]) and np.all(np.isfinite(got[1]))
+
+
+@pytest.mark.parametrize("mesh", [32, 27, 256])
+def test_unkeyable_particles_leave_the_state_as_it_was(mesh):
+    """Meshes whose deposit form the device picks (five-pass and cuFFT) and one where the
+    host reads the densest bucket between the sort and the deposit."""
+    L, pos = state(n=4096, seed=6)
+    noise = np.random.default_rng(6).standard_normal(16 ** 3)
+    noise[5] = np.nan
+    with hb.PMSolver(hb.MeshGeometry(L, mesh), hb.PMForceMethod.pure_pm(False)) as s:
+        s.upload(*pos, uniform_mass=1.0)
+        s.solve_forces()
+        want = s.download()
+        ic.lpt_on_device(s, noise, 16, 0.05, 1.0)
+        before = s.download(acc=False)
+        for _ in range(2):
+            with pytest.raises(ValueError, match="finite"):
+                s.solve_forces()
+            after = s.download(acc=False)
+            for k in before:
+                assert np.array_equal(before[k], after[k], equal_nan=True), k
+        s.upload(*pos, uniform_mass=1.0)
+        s.solve_forces()
+        got = s.download()
+    for k in ("ax", "ay", "az"):
+        assert np.array_equal(got[k], want[k]), k
