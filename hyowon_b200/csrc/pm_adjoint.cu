@@ -739,7 +739,10 @@ public:
         return c.box_size == cfg_.box_size && c.mesh_size == cfg_.mesh_size
             && c.n_side == cfg_.n_side && c.precision == cfg_.precision;
     }
-    void set_config(const VjpConfig& c) { cfg_ = c; }
+    void set_config(const VjpConfig& c, size_t potential_limit) {
+        cfg_ = c;
+        potential_limit_ = potential_limit;
+    }
 
     // Gives the work arrays of a run back; the next run takes them again.
     void trim() {
@@ -880,7 +883,7 @@ public:
             const size_t rest = arena_.count(layout);
             size_t free_b = 0, total_b = 0;
             const size_t need = (S + 1) * phi_stride * sizeof(R);
-            keep = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess
+            keep = need <= potential_limit_ && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess
                 && rest <= free_b + arena_.capacity()
                 && need + (size_t(1) << 30) < (free_b + arena_.capacity() - rest) / 2;
         }
@@ -1047,6 +1050,7 @@ private:
     R* p_[3] = {};
     R* acc_[3] = {};
     uint64_t solves_ = 0, vjps_ = 0;
+    size_t potential_limit_ = SIZE_MAX;
     Arena fixed_;       // what the engine keeps: meshes, spectrum, particle state
     Arena arena_;       // a run's work arrays
     LptWork lpt_;
@@ -1060,6 +1064,7 @@ thread_local std::string g_adj_err;
 struct Cache {
     Engine<double>* e64 = nullptr;
     Engine<float>* e32 = nullptr;
+    size_t potential_limit = SIZE_MAX;
     ~Cache() {
         delete e64;
         delete e32;
@@ -1074,6 +1079,13 @@ void trim_cache(Cache* c) {
     if (c->e32) c->e32->trim();
 }
 
+int limit_potentials(Cache** c, size_t bytes) {
+    if (!*c) *c = new (std::nothrow) Cache();
+    if (!*c) return HYOWON_ENOMEM;
+    (*c)->potential_limit = bytes;
+    return HYOWON_OK;
+}
+
 int run_cached(Cache** cache, const VjpConfig& cfg, cudaStream_t s, const double* noise,
                const double* target_delta, double* loss, double* grad_noise,
                double* final_delta, double* timings, std::string* err) {
@@ -1086,7 +1098,7 @@ int run_cached(Cache** cache, const VjpConfig& cfg, cudaStream_t s, const double
                 c->e64 = nullptr;
             }
             if (!c->e64) c->e64 = new Engine<double>(cfg, s);
-            c->e64->set_config(cfg);
+            c->e64->set_config(cfg, c->potential_limit);
             c->e64->run(noise, target_delta, loss, grad_noise, final_delta, timings);
         } else {
             if (c->e32 && !c->e32->same_geometry(cfg)) {
@@ -1094,7 +1106,7 @@ int run_cached(Cache** cache, const VjpConfig& cfg, cudaStream_t s, const double
                 c->e32 = nullptr;
             }
             if (!c->e32) c->e32 = new Engine<float>(cfg, s);
-            c->e32->set_config(cfg);
+            c->e32->set_config(cfg, c->potential_limit);
             c->e32->run(noise, target_delta, loss, grad_noise, final_delta, timings);
         }
     } catch (const Fail& f) {

@@ -1586,6 +1586,11 @@ int hyowon_pm_debug_set_wait_limit(hyowon_pm_t h, unsigned polls) {
     return HYOWON_OK;
 }
 
+int hyowon_pm_debug_limit_potentials(hyowon_pm_t h, uint64_t bytes) {
+    if (!h) return HYOWON_EINVAL;
+    return hyowon::adj::limit_potentials(&h->adj, static_cast<size_t>(bytes));
+}
+
 int hyowon_pm_debug_tree_allocations(hyowon_pm_t h, uint64_t* count) {
     if (!h || !count) return HYOWON_EINVAL;
     *count = tree::workspace_allocations(h->tree_ws);

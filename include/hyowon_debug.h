@@ -31,6 +31,11 @@ int hyowon_pm_debug_set_wait_limit(hyowon_pm_t h, unsigned polls);
  * plus delta units. 0 restores the exact target. */
 int hyowon_pm_debug_offset_mass_target(hyowon_pm_t h, double delta);
 
+/* Device bytes that hyowon_pm_vjp may keep the forward potentials in (by default up to
+ * half the free memory). Without room for them the reverse pass solves again for
+ * the force of each state, as it does for meshes and schedules too large to keep. */
+int hyowon_pm_debug_limit_potentials(hyowon_pm_t h, uint64_t bytes);
+
 /* cudaMalloc calls made so far for the octree's work arrays of this handle (a
  * clustering run makes none from its third solve on). */
 int hyowon_pm_debug_tree_allocations(hyowon_pm_t h, uint64_t* count);

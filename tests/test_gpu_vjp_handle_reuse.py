@@ -6,10 +6,13 @@ hyowon_vjp_1lpt_pm of the same inputs: the two run the same kernels and differ
 only in the order of the deposit's atomics (1e-11 relative in binary64, 2e-3 in
 FP32, the spread of repeated stateless calls times ten).
 """
+import ctypes
+
 import numpy as np
 import pytest
 
 import hyowon_b200 as hb
+from hyowon_b200 import _native as nat
 from hyowon_b200 import adjoint, ic
 
 pytestmark = pytest.mark.gpu
@@ -96,3 +99,26 @@ def test_counts_are_those_of_the_call(precision):
         for _ in range(3):
             d.loss_and_grad(noise, target)
             assert {k: d.last_timings[k] for k in want} == want
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("N", [32, 27])
+@pytest.mark.parametrize("steps,every", [(4, 1), (5, 2), (6, 4), (3, 5)])
+def test_gradient_without_room_for_the_potentials(N, steps, every, precision):
+    """The reverse pass that solves again for each state against the one that kept the
+    forward potentials, on the five-pass solve and on cuFFT, with checkpoints at every
+    step, between and none but the first: the same kernels, so equal to the order of the
+    deposit's atomics; a solve more for every step shows which ran."""
+    box, n = 60.0, 16
+    noise, target = inputs(n, N, steps + N)
+    args = (box, n, N, 0.05, steps, precision, every)
+    with hb.PMSolver(hb.MeshGeometry(box, N), hb.PMForceMethod.pure_pm(False), precision) as s:
+        d = adjoint.DifferentiablePM(*args, solver=s)
+        want = d.loss_and_grad(noise, target)
+        assert d.last_timings["force_solves"] == steps + 1
+        assert nat.lib().hyowon_pm_debug_limit_potentials(s.handle, ctypes.c_uint64(0)) == 0
+        got = d.loss_and_grad(noise, target)
+        assert d.last_timings["force_solves"] == 2 * steps + 1
+    tol = TOL[precision]
+    assert abs(got[0] - want[0]) <= tol * abs(want[0])
+    assert np.linalg.norm(got[1] - want[1]) <= tol * np.linalg.norm(want[1])
