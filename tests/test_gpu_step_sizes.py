@@ -6,9 +6,10 @@ device picks), the bucket scan runs in one block up to four tiles of 4096 counts
 in two kernels above, and the densest bucket is found by the scan. One KDK step of
 each size against the oracle: binary64 positions to 1e-12 of a cell, forces to 1e-12
 of the largest; the FP32 form's forces to 1e-4 of the largest (its bar) and what
-the deposit's weights cut off (B bits of each fraction, where 8 n 2^(3B) < 2^63 in the
-worst case of all particles in one bucket, shift mass by up to 2^-B of a cell on three
-axes, and the force changes by at most twice the largest within a cell), its
+the deposit's weights cut off (B bits of each fraction, the most up to 16 for which
+8 c 2^(3B) < 2^63, c the densest bucket of the states deposited; cutting shifts mass by
+up to 2^-B of a cell on three axes, and the force changes by at most twice the largest
+within a cell: 9e-5 at 16 bits), its
 positions to what that error of the opening kick drifts, the FP32 rounding of the
 momenta and two units of the fixed-point coordinates, and the force after the drift
 also to what that shift of the particle and of its sources changes.
@@ -30,6 +31,21 @@ def state(n, L, clustered, seed):
     return p, rng.normal(0, 1.0, (3, n))
 
 
+def fraction_bits(N, n, L, states):
+    """B of the densest bucket (2^shift consecutive cells, some eight particles)."""
+    shift = 0
+    while (N ** 3 >> (shift + 1)) * 8 >= n and N ** 3 >> (shift + 1):
+        shift += 1
+    densest = 0
+    for p in states:
+        i, j, k = (np.minimum((np.mod(c, L) / L * N).astype(np.int64), N - 1) for c in p)
+        densest = max(densest, int(np.bincount((((i * N) + j) * N + k) >> shift).max()))
+    bits = 16
+    while 8 * densest << 3 * bits > 2 ** 63 - 1:
+        bits -= 1
+    return bits
+
+
 # buckets + 1 = 4097 at (64, 32768), 16385 (five tiles) at (128, 100000), 5 at (12, 40)
 @pytest.mark.parametrize("clustered", [False, True])
 @pytest.mark.parametrize("N,n", [(12, 40), (16, 5000), (31, 3000), (32, 4096), (33, 7), (48, 20000),
@@ -43,7 +59,7 @@ def test_one_step_against_the_oracle(oracle, N, n, clustered):
     scale0 = max(float(np.max(np.abs(ref[a]))) for a in ("ax", "ay", "az"))
     drift = oracle.kdk_step(L, N, ref, K1, D, K2, uniform_mass=m)
     scale = max(float(np.max(np.abs(ref[a]))) for a in ("ax", "ay", "az"))
-    bits = min(16, int((60 - np.log2(n)) // 3))
+    bits = fraction_bits(N, n, L, [(x, y, z), (ref["x"], ref["y"], ref["z"])])
     for precision, tol in (("fp64", 1e-12), ("fp32", 1e-4 + 6.0 * 2.0 ** -bits)):
         with hb.PMSolver(hb.MeshGeometry(L, N), hb.PMForceMethod.pure_pm(False), precision) as s:
             s.upload(x, y, z, px, py, pz, uniform_mass=m)
