@@ -3,8 +3,12 @@
 A handle keeps the adjoint's plans and work arrays between calls and gives them
 back before other calls that allocate. Each call must equal the stateless
 hyowon_vjp_1lpt_pm of the same inputs: the two run the same kernels and differ
-only in the order of the deposit's atomics (1e-11 relative in binary64, 2e-3 in
-FP32, the spread of repeated stateless calls times ten).
+only in the order of the deposit's atomics. In binary64 that is 1e-11 relative. In
+FP32 the gradients of two stateless calls differ by 3e-6 (99 of 100 by less than
+1e-5), but in up to 3 of 100 pairs a particle comes to lie on the other side of a
+cell face, where the force's derivative jumps: one of 4096 particles, a 64th of the
+gradient's norm (1.9e-2 seen). So an FP32 gradient may differ by 0.1, and must agree
+to 2e-4 for one of three seeds; a wrong gradient differs by its own size in all.
 """
 import ctypes
 
@@ -17,7 +21,8 @@ from hyowon_b200 import adjoint, ic
 
 pytestmark = pytest.mark.gpu
 
-TOL = {"fp64": 1e-11, "fp32": 2e-3}
+LOSS = {"fp64": 1e-11, "fp32": 1e-5}
+SEEDS = {"fp64": (0,), "fp32": (0, 1000, 2000)}
 
 
 def inputs(n, N, seed):
@@ -25,14 +30,29 @@ def inputs(n, N, seed):
     return rng.standard_normal(n ** 3), 0.3 * rng.standard_normal(N ** 3)
 
 
+def assert_agree(precision, both):
+    """both(offset of the seed): two (loss, gradient) pairs."""
+    for offset in SEEDS[precision]:
+        got, ref = both(offset)
+        assert abs(got[0] - ref[0]) <= LOSS[precision] * abs(ref[0])
+        off = np.linalg.norm(got[1] - ref[1]) / np.linalg.norm(ref[1])
+        if precision == "fp64":
+            assert off <= 1e-11
+        else:
+            assert off <= 0.1
+            if off <= 2e-4:
+                return
+    assert precision == "fp64", "three gradients in a row differ"
+
+
 def check(solver, box, n, N, steps, every, precision, seed):
-    noise, target = inputs(n, N, seed)
     args = (box, n, N, 0.05, steps, precision, every)
-    ref = adjoint.DifferentiablePM(*args).loss_and_grad(noise, target)
-    got = adjoint.DifferentiablePM(*args, solver=solver).loss_and_grad(noise, target)
-    tol = TOL[precision]
-    assert abs(got[0] - ref[0]) <= tol * abs(ref[0])
-    assert np.linalg.norm(got[1] - ref[1]) <= tol * np.linalg.norm(ref[1])
+
+    def both(offset):
+        noise, target = inputs(n, N, seed + offset)
+        return (adjoint.DifferentiablePM(*args, solver=solver).loss_and_grad(noise, target),
+                adjoint.DifferentiablePM(*args).loss_and_grad(noise, target))
+    assert_agree(precision, both)
 
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
@@ -82,7 +102,7 @@ def test_large_lattice_leaves_the_engine_alone():
         first = d.loss(noise, target)
         held = free - torch.cuda.mem_get_info()[0]
         assert abs(held - 48 * n ** 3) <= 256 << 20, held
-        assert abs(d.loss(noise, target) - first) <= TOL["fp32"] * abs(first)
+        assert abs(d.loss(noise, target) - first) <= LOSS["fp32"] * abs(first)
 
 
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
@@ -107,18 +127,19 @@ def test_counts_are_those_of_the_call(precision):
 def test_gradient_without_room_for_the_potentials(N, steps, every, precision):
     """The reverse pass that solves again for each state against the one that kept the
     forward potentials, on the five-pass solve and on cuFFT, with checkpoints at every
-    step, between and none but the first: the same kernels, so equal to the order of the
-    deposit's atomics; a solve more for every step shows which ran."""
+    step, between and none but the first; a solve more for every step shows which ran."""
     box, n = 60.0, 16
-    noise, target = inputs(n, N, steps + N)
     args = (box, n, N, 0.05, steps, precision, every)
     with hb.PMSolver(hb.MeshGeometry(box, N), hb.PMForceMethod.pure_pm(False), precision) as s:
         d = adjoint.DifferentiablePM(*args, solver=s)
-        want = d.loss_and_grad(noise, target)
-        assert d.last_timings["force_solves"] == steps + 1
-        assert nat.lib().hyowon_pm_debug_limit_potentials(s.handle, ctypes.c_uint64(0)) == 0
-        got = d.loss_and_grad(noise, target)
-        assert d.last_timings["force_solves"] == 2 * steps + 1
-    tol = TOL[precision]
-    assert abs(got[0] - want[0]) <= tol * abs(want[0])
-    assert np.linalg.norm(got[1] - want[1]) <= tol * np.linalg.norm(want[1])
+
+        def run(noise, target, limit, solves):
+            assert nat.lib().hyowon_pm_debug_limit_potentials(s.handle, ctypes.c_uint64(limit)) == 0
+            r = d.loss_and_grad(noise, target)
+            assert d.last_timings["force_solves"] == solves
+            return r
+
+        def both(offset):
+            noise, target = inputs(n, N, steps + N + offset)
+            return (run(noise, target, 0, 2 * steps + 1), run(noise, target, 1 << 40, steps + 1))
+        assert_agree(precision, both)
