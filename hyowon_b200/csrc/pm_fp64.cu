@@ -220,9 +220,10 @@ constexpr int kTileThreads = 256;
 // W >= kOneWordMinW, a single 64-bit word per cell holds the sum of terms
 // quantised to q = rint(t 2^(W-1-e)): a quantum of 2^(e+1-W) <= 2^(e-54), below
 // half the binary64 spacing of a full-weight term (t < 2^e). Cell sums stay
-// below 2^63. Denser states use the exact two-word (hi/lo) sums. The host reads
-// the densest bucket count before the deposit and launches the form that
-// applies (the kernel checks the same condition on the device).
+// below 2^63. Denser states use the exact two-word (hi/lo) sums. Above 128^3 cells
+// the host reads the densest bucket count before the deposit and launches the form
+// that applies; up to there both are launched, and the one that does not apply
+// returns (every block checks the condition on the device).
 constexpr int kOneWordMinW = 55;
 // Two words: a hi part is below 2^(62-W) <= c/2 for c = 8 max_bucket
 // contributors, so hi sums stay below c^2 / 2 < 2^64 while c < 2^32, i.e.

@@ -34,12 +34,6 @@ size_t scan_tmp_elements(uint32_t n_buckets);
 // value is folded into it (atomicMax; the caller zeroes it).
 int launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n,
                           uint32_t* tmp, cudaStream_t s, uint32_t* most = nullptr);
-void launch_scatter_u32(uint32_t n, const uint32_t* key, const uint32_t* rank,
-                        const uint32_t* offset, const uint32_t* src, uint32_t* dst,
-                        const unsigned int* status, cudaStream_t s);
-void launch_scatter_f64(uint32_t n, const uint32_t* key, const uint32_t* rank,
-                        const uint32_t* offset, const double* src, double* dst,
-                        const unsigned int* status, cudaStream_t s);
 void launch_unpermute_f64(uint32_t n, const uint32_t* id, const double* src, double* dst,
                           cudaStream_t s);
 // Up to eight arrays at once: dst[a][id[i]] = src[a][i].
@@ -78,7 +72,8 @@ void launch_deposit_f64(uint32_t n, const ParticlesF64& p, const double* mass,
 // no zeroing needed. Needs the bucket offsets of the deposited set in w, the
 // cell order `order` (or null when the arrays are in cell order), the largest
 // bucket count in *max_count (and its value on the host, which picks the
-// kernel; null: both forms are launched and the device's value picks) and e_max = deposit_mass_exponent_f64(max mass).
+// kernel; null: both forms are launched and the device's value picks) and
+// e_max = deposit_mass_exponent_f64(max mass).
 int deposit_mass_exponent_f64(double max_mass);
 // With `modes` non-null (a power-of-two mesh of 32 to 2048), the tiles are
 // transformed along z and stored to that chunked half spectrum (twiddles `tw`)

@@ -230,18 +230,6 @@ int launch_exclusive_scan(const uint32_t* in, uint32_t* out, uint32_t n, uint32_
     return 2 + inner;
 }
 
-void launch_scatter_u32(uint32_t n, const uint32_t* key, const uint32_t* rank,
-                        const uint32_t* offset, const uint32_t* src, uint32_t* dst,
-                        const unsigned int* status, cudaStream_t s) {
-    if (n == 0) return;
-    ScatterArrays a{};
-    a.src_u[0] = src;
-    a.dst_u[0] = dst;
-    a.n_f64 = 0;
-    a.n_u32 = 1;
-    k_scatter<<<blocks_for(n, 256), 256, 0, s>>>(n, key, rank, offset, a, status);
-}
-
 void launch_scatter_multi(uint32_t n, const uint32_t* key, const uint32_t* rank,
                           const uint32_t* offset, int n_f64, const double* const* src,
                           double* const* dst, int n_u32, const uint32_t* const* src_u,

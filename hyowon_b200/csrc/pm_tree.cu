@@ -16,7 +16,7 @@
 //      level counts and one scan number the nodes level by level;
 //   4. node mass and COM from exact 64-bit prefix sums of 2^-40 L fixed-point
 //      coordinates (no summation-order error).
-// Walk: one warp per group of G targets (G of 1, 8, 16 or 32, neighbours in key
+// Walk: one warp per group of G targets (G of 1, 4, 8 or 16, neighbours in key
 // order). The 32 lanes classify 32 nodes at a time against the group's bounding
 // box: dropped for every target, opened for every target, a monopole for every
 // target, or undecided, in which case each target decides for itself in
@@ -567,11 +567,14 @@ __device__ __forceinline__ double pair_factor(double r2, double eps2, double inv
 // with one lane per target ran with 11 of 32 lanes active, and each lane
 // classified every node its warp reached in binary64; here a node costs one lane a
 // few integer and FP32 operations for the whole group.
-// 24 warps per SM (80 registers, no spill in the forms that run): 28 and 20 measured
-// 34.2 / 33.6 / 34.8 ms on 2.1M clustered sources at G = 16.
+// Registers for 24 warps per SM (80; 8 to 44 bytes of spill in the closed form and at
+// degree 36, none in the others); caps for 28 and 20 measured 34.2 / 33.6 / 34.8 ms on
+// 2.1M clustered sources at G = 16. Shared memory holds 23 of these one-warp
+// blocks per SM at G = 16 and 17 at G = 1, 4 and 8.
 constexpr int kWalkWarps = 24;
 template <int G>
 struct WalkShape {
+    static_assert(G >= 1 && G <= 16, "lane and mask layout");
     static constexpr int S = 32 / G;                  // lanes per target
     static constexpr int cap = S < 4 ? 32 * S : 128;  // list entries, >= 32
     static constexpr int per_lane = cap / S;          // one bit each of a 32-bit word
@@ -590,7 +593,7 @@ k_walk(uint32_t n_targets, const uint32_t* __restrict__ tslot, const double* __r
        unsigned long long* __restrict__ counters, unsigned int* status) {
     using Shape = WalkShape<G>;
     constexpr int S = Shape::S, CAP = Shape::cap, PER = Shape::per_lane;
-    constexpr uint32_t kGroup = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+    constexpr uint32_t kGroup = (1u << G) - 1u;
     constexpr unsigned kAll = 0xffffffffu;
     __shared__ double ex[CAP], ey[CAP], ez[CAP], ew[CAP];  // entry position (the group's image), G m
     __shared__ float4 erel[CAP];              // (position - group centre) / r_cut, target mask
@@ -692,7 +695,7 @@ k_walk(uint32_t n_targets, const uint32_t* __restrict__ tslot, const double* __r
     if (lane == 0) {
         run_first[0] = 0;
         run_count[0] = 1;
-        run_mask[0] = n_here == 32u ? kAll : (1u << n_here) - 1u;
+        run_mask[0] = (1u << n_here) - 1u;
     }
     int sp = 1;
     __syncwarp();
@@ -1431,7 +1434,7 @@ int run(const hyowon_treepm_params& P, uint32_t n, const double* x, const double
         sm = mem.get<double>(n);
         k_gather_masses<<<nb(n), kT, 0, s>>>(n, sval, masses, sm);
     }
-    // nodes, level by level
+    // nodes: how many of each level, then all in one sweep
     const uint32_t n_node_tiles = nb(n);
     const uint32_t n_counts = kLevels * n_node_tiles + 1;
     uint32_t* level_hist = mem.get<uint32_t>(n_counts);
