@@ -547,6 +547,7 @@ def run_treepm(args, rank, emit=True):
     for form in ("fp64", "fp32"):
         with hb.PMSolver(hb.MeshGeometry(L, N), hb.PMForceMethod.treepm_long_range(r_s), form) as s:
             s.upload(st["x"], st["y"], st["z"], st["px"], st["py"], st["pz"], uniform_mass=m)
+            s.treepm_short_forces(0.5, eps, 4.5 * r_s)   # takes the work arrays
             sx, sy, sz, info = s.treepm_short_forces(0.5, eps, 4.5 * r_s)
             s.set_treepm_short_range(0.5, eps, 4.5 * r_s)
             s.solve_forces()

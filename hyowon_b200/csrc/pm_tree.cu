@@ -1359,7 +1359,8 @@ void launch_walk(const WalkArgs& A, const PairForm& form, int group, cudaStream_
 // Targets a warp takes. A larger group shares the node tests among more targets
 // but has a larger box, so more undecided nodes and rejected pairs, and fewer
 // warps. Measured walk ms at G = 4 / 8 / 16 (clustered sources, every source a
-// target): 30,000: 0.87 / 0.96 / 1.36; 262,144: 4.7 / 4.0 / 4.9; 2.1M: 39 / 30 / 25;
+// target; binary64 with the pair factor at degree 20, 26.6 instead of 25.4 at 28):
+// 30,000: 0.87 / 0.96 / 1.36; 262,144: 4.7 / 4.0 / 4.9; 2.1M: 39 / 30 / 25;
 // 16.8M: 290 / 213 / 166 (in Morton order 25 to 30% more: 4.9, 32 and 191 at the
 // chosen G; one lane per target: 15, 48, 168 and 696). Targets that are a sample of
 // the sources lie further apart: of 2.1M sources, 4,096 targets take 0.66 ms at
