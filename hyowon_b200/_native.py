@@ -117,6 +117,8 @@ _SIGS = {
     "hyowon_pm_set_treepm_short_range": (c_int, [c_void_p, c_double, c_double, c_double]),
     "hyowon_pm_debug_set_wait_limit": (c_int, [c_void_p, ctypes.c_uint]),
     "hyowon_pm_debug_offset_mass_target": (c_int, [c_void_p, c_double]),
+    "hyowon_pm_debug_limit_potentials": (c_int, [c_void_p, c_u64]),
+    "hyowon_pm_debug_tree_allocations": (c_int, [c_void_p, P_u64]),
     "hyowon_pm_treepm_short_forces": (c_int, [c_void_p, c_double, c_double, c_double]
                                       + [P_double] * 4),
     "hyowon_cic_deposit_noalloc": (c_int, [c_double, c_u64, c_u64, c_void_p, c_void_p,

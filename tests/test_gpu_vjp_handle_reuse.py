@@ -10,8 +10,6 @@ cell face, where the force's derivative jumps: one of 4096 particles, a 64th of 
 gradient's norm (1.9e-2 seen). So an FP32 gradient may differ by 0.1, and must agree
 to 2e-4 for one of three seeds; a wrong gradient differs by its own size in all.
 """
-import ctypes
-
 import numpy as np
 import pytest
 
@@ -134,7 +132,7 @@ def test_gradient_without_room_for_the_potentials(N, steps, every, precision):
         d = adjoint.DifferentiablePM(*args, solver=s)
 
         def run(noise, target, limit, solves):
-            assert nat.lib().hyowon_pm_debug_limit_potentials(s.handle, ctypes.c_uint64(limit)) == 0
+            assert nat.lib().hyowon_pm_debug_limit_potentials(s.handle, limit) == 0
             r = d.loss_and_grad(noise, target)
             assert d.last_timings["force_solves"] == solves
             return r
